@@ -124,3 +124,34 @@ def test_noalloc_sweep_rejects_problems_beyond_its_scratch(built):
         check(lib().tycho_sweeper_sweep_noalloc(sw._h, 0, None, C.c_void_p(psi.data_ptr()), None))
     assert e.value.status == 1 and "at most 16777216" in str(e.value)
     sw.close()
+
+
+@pytest.mark.parametrize("n,sn,G", [(6, 10, 5), (15, 6, 5), (7, 8, 7), (6, 8, 3)])
+def test_noalloc_sweep_keeps_to_the_callers_rows(built, n, sn, G):
+    """The default FP32 form keeps its own psi in padded rows for some odd group
+    counts (5 and 7 here); the caller's buffers have rows of the G groups, and
+    nothing behind them is touched."""
+    import torch
+    import tycho2_b200 as ty
+    from tycho2_b200._capi import check
+
+    mesh = ty.TychoMesh.kuhn_cube(n, 0.05, 31, 1.0)
+    sw = ty.SweeperCuda(mesh, sn, G, fp32=True)
+    rng = np.random.default_rng(n + G)
+    st = rng.lognormal(0.0, 0.5, mesh.n_cells)
+    sw.set_cross_sections(st, np.zeros(mesh.n_cells))
+    q = rng.uniform(0.5, 1.0, sw.phi_shape)
+    src = np.ascontiguousarray(np.broadcast_to(q[:, None, :, :], sw.psi_shape))
+    psi_ref = np.empty(sw.psi_shape)
+    sw.sweep(psi_ref, src)
+    stream = torch.cuda.current_stream()
+    size, guard = int(np.prod(sw.psi_shape)), 1 << 16
+    for precision, dtype in ((1, torch.float32), (0, torch.float64)):
+        iso = torch.tensor(q, dtype=dtype, device="cuda").contiguous()
+        buf = torch.full((size + guard,), -3.0, dtype=dtype, device="cuda")
+        stream.synchronize()
+        check(_noalloc(sw, precision, iso, buf, stream))
+        assert bool((buf[size:] == -3.0).all())
+        out = buf[:size].cpu().numpy().astype(np.float64).reshape(sw.psi_shape)
+        _check(out, psi_ref, precision, "precision %d" % precision)
+    sw.close()

@@ -654,6 +654,13 @@ LevelArgs Sweeper::level_args(int prec, const void *iso, const double *qang, voi
     p.solver = (uint32_t)solver_;
     p.zero_row = prec ? 2 * zero_row_ : zero_row_;
     p.scalar = 0;
+    return p;
+}
+
+LevelArgs Sweeper::form_args(int prec, bool has_iso, const double *qang) const
+{
+    const void *iso = has_iso ? (prec ? (const void *)d_iso32_ : (const void *)d_iso_) : nullptr;
+    LevelArgs p = level_args(prec, iso, qang, d_psi_);
     if (prec && block_[1]) {
         p.G = block_rows_.groups;
         p.vg = block_rows_.vg;
@@ -762,8 +769,7 @@ int Sweeper::ensure_form_records(int prec, std::string &err)
 
 cudaError_t Sweeper::enqueue_chains(int prec, bool has_iso, const double *qang)
 {
-    const void *iso = has_iso ? (prec ? (const void *)d_iso32_ : (const void *)d_iso_) : nullptr;
-    const LevelArgs p = level_args(prec, iso, qang, d_psi_);
+    const LevelArgs p = form_args(prec, has_iso, qang);
     return prec ? launch_chains<float>(chains_[1], p, d_crec_[1], d_chain_off_, sched_.n_levels, (uint32_t)A_,
                                        stream_)
                 : launch_chains<double>(chains_[0], p, d_crec_[0], d_chain_off_, sched_.n_levels, (uint32_t)A_,
@@ -921,9 +927,8 @@ int Sweeper::levels(int prec, bool has_iso, const double *qang, cudaEvent_t beg,
 cudaError_t Sweeper::enqueue_levels(int prec, bool has_iso, const double *qang)
 {
     if (chains_[prec ? 1 : 0].threads) return enqueue_chains(prec, has_iso, qang);
-    const void *iso = has_iso ? (prec ? (const void *)d_iso32_ : (const void *)d_iso_) : nullptr;
     const LaunchShape &sh = shape_[prec ? 1 : 0];
-    const LevelArgs p = level_args(prec, iso, qang, d_psi_);
+    const LevelArgs p = form_args(prec, has_iso, qang);
     cudaError_t le = cudaSuccess;
     const int S = sh.streams;
     if (S > 1) le = cudaEventRecord(fork_, stream_);

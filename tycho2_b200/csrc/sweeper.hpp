@@ -206,7 +206,12 @@ private:
     void drop_si_graph();
     // Reads (and clears) the dataflow schedule's device error word.
     int check_device_error(std::string &err);
+    // The arguments of a sweep over rows [v][g] of the sweeper's groups: the
+    // caller's buffers, and the resident ones of every configured shape.
     LevelArgs level_args(int prec, const void *iso, const double *qang, void *psi) const;
+    // The same for the resident psi and source in the rows of the form in use
+    // (the default FP32 form keeps them as blocks, padded for some odd counts).
+    LevelArgs form_args(int prec, bool has_iso, const double *qang) const;
     int launch_dataflow_shape(int prec, const LevelArgs &p, const DataflowArgs &df, cudaStream_t s,
                               std::string &err);
     // r_out (nullable): on return b - (I - K) x from the last cycle's Arnoldi
