@@ -87,7 +87,7 @@ Sweeper::~Sweeper()
                     d_w_, d_sigs_, d_scat_, d_qiso_, d_qang_, d_src_, d_iso_, d_iso32_, d_psi_,
                     d_phi_, d_r_, d_tmp_, d_V_, d_h_, d_flush_, d_done_, d_ctl_, d_rec_[0], d_rec_[1],
                     d_level_off_, d_barrier_, d_crec_[0], d_crec_[1], d_flags_, d_adj32_, d_psi_prev_,
-                    d_chain_pos_, d_chain_off_};
+                    chain_.pos, chain_.off};
     for (void *b : bufs) dev_free(b, stream_);
     for (auto &kv : links_) {
         dev_free(kv.second.d_send_row, stream_);
@@ -162,9 +162,7 @@ int Sweeper::set_work_order(int order, std::string &err)
     // everything kept per item position is stale
     rec_valid_[0] = rec_valid_[1] = false;
     crec_valid_[0] = crec_valid_[1] = false;
-    dev_free(d_chain_pos_, stream_);
-    dev_free(d_chain_off_, stream_);
-    d_chain_pos_ = d_chain_off_ = nullptr;
+    chain_.drop([&](uint32_t *p) { dev_free(p, stream_); });
     for (auto &kv : graphs_) cudaGraphExecDestroy(kv.second.exec);
     graphs_.clear();
     drop_si_graph();
@@ -679,7 +677,7 @@ int Sweeper::device_view(int prec, DeviceView &v, std::string &err, bool compact
     TY_CUDA(cudaSetDevice(device_));
     TY_CHECK(ensure_records(prec, true, err, compact, chain));
     TY_CUDA(cudaStreamSynchronize(stream_));
-    v.chain_off = d_chain_off_;
+    v.chain_off = chain_.off;
     v.rec = compact ? d_crec_[prec ? 1 : 0] : d_rec_[prec ? 1 : 0];
     v.psi = d_psi_;
     v.iso = d_iso_;
@@ -725,7 +723,7 @@ int Sweeper::ensure_records(int prec, bool need_filled, std::string &err, bool c
     if (!valid && have_xs_) {
         const LevelArgs p = level_args(prec, nullptr, nullptr, d_psi_);
         const uint64_t n = chain ? sched_.n_items : sched_.n_padded;
-        const uint32_t *pos = chain ? d_chain_pos_ : nullptr;
+        const uint32_t *pos = chain ? chain_.pos : nullptr;
         if (compact)
             TY_CUDA(prec ? launch_compact_records<float>(p, n, pos, buf, stream_)
                          : launch_compact_records<double>(p, n, pos, buf, stream_));
@@ -742,17 +740,21 @@ int Sweeper::ensure_records(int prec, bool need_filled, std::string &err, bool c
 
 int Sweeper::ensure_chain_plan(std::string &err)
 {
-    if (d_chain_pos_) return kOk;
     std::vector<uint64_t> seg;
-    TY_CHECK(angle_chunks_device(d_items_, sched_.n_padded, d_level_off_, sched_.n_levels, (uint32_t)A_,
-                                 (uint32_t)A_, &d_chain_pos_, seg, stream_, err));
-    const size_t nl = sched_.n_levels;
-    std::vector<uint32_t> off((size_t)A_ * (nl + 2));
-    for (size_t a = 0; a < (size_t)A_; ++a)
-        for (size_t l = 0; l < nl + 2; ++l) off[a * (nl + 2) + l] = (uint32_t)seg[a * nl + std::min(l, nl)];
-    TY_CUDA(upload(d_chain_off_, off.data(), off.size(), stream_));
-    TY_CUDA(cudaStreamSynchronize(stream_));
-    return kOk;
+    auto positions = [&](uint32_t *&pos) {
+        return angle_chunks_device(d_items_, sched_.n_padded, d_level_off_, sched_.n_levels, (uint32_t)A_,
+                                   (uint32_t)A_, &pos, seg, stream_, err);
+    };
+    auto offsets = [&](uint32_t *&dst) -> int {
+        const size_t nl = sched_.n_levels;
+        std::vector<uint32_t> off((size_t)A_ * (nl + 2));
+        for (size_t a = 0; a < (size_t)A_; ++a)
+            for (size_t l = 0; l < nl + 2; ++l) off[a * (nl + 2) + l] = (uint32_t)seg[a * nl + std::min(l, nl)];
+        TY_CUDA(upload(dst, off.data(), off.size(), stream_));
+        TY_CUDA(cudaStreamSynchronize(stream_));
+        return kOk;
+    };
+    return chain_.make(positions, offsets, [&](uint32_t *p) { dev_free(p, stream_); });
 }
 
 int Sweeper::ensure_form_records(int prec, std::string &err)
@@ -770,9 +772,9 @@ int Sweeper::ensure_form_records(int prec, std::string &err)
 cudaError_t Sweeper::enqueue_chains(int prec, bool has_iso, const double *qang)
 {
     const LevelArgs p = form_args(prec, has_iso, qang);
-    return prec ? launch_chains<float>(chains_[1], p, d_crec_[1], d_chain_off_, sched_.n_levels, (uint32_t)A_,
+    return prec ? launch_chains<float>(chains_[1], p, d_crec_[1], chain_.off, sched_.n_levels, (uint32_t)A_,
                                        stream_)
-                : launch_chains<double>(chains_[0], p, d_crec_[0], d_chain_off_, sched_.n_levels, (uint32_t)A_,
+                : launch_chains<double>(chains_[0], p, d_crec_[0], chain_.off, sched_.n_levels, (uint32_t)A_,
                                         stream_);
 }
 

@@ -11,6 +11,7 @@
 
 #include <cuda_runtime.h>
 
+#include "chain_plan.hpp"
 #include "device_ops.hpp"
 #include "mesh.hpp"
 #include "schedule.hpp"
@@ -292,9 +293,8 @@ private:
     // whether they are in chain order (direction, level) instead of level
     // order: one buffer, filled again when the other order is swept
     bool crec_chain_[2] = {false, false};
-    // Direction chains (sweep_chains.cuh): the schedule positions in chain
-    // order and each direction's level offsets (made on first use).
-    uint32_t *d_chain_pos_ = nullptr, *d_chain_off_ = nullptr;
+    // Direction chains (sweep_chains.cuh): made on first use.
+    ChainPlan chain_;
     int ensure_chain_plan(std::string &err);
     // The records of the form in use, allocated and filled.
     int ensure_form_records(int prec, std::string &err);
