@@ -50,7 +50,11 @@ cudaError_t dev_malloc(void **p, size_t bytes, cudaStream_t s)
     cudaMemPool_t pool;
     cudaError_t e = pool_of_current(&pool);
     if (e != cudaSuccess) return e;
-    return cudaMallocFromPoolAsync(p, bytes ? bytes : 1, pool, s);
+    e = cudaMallocFromPoolAsync(p, bytes ? bytes : 1, pool, s);
+    // the caller has the status; left behind, it would be taken for the error
+    // of the next launch, that of a form that needs less memory
+    if (e == cudaErrorMemoryAllocation) cudaGetLastError();
+    return e;
 }
 
 void dev_free(void *p, cudaStream_t s)

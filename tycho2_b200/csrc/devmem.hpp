@@ -12,6 +12,7 @@ namespace tycho {
 
 // Allocates `bytes` (at least 1) on the current device, ordered on stream s;
 // the memory may be used on other streams once s has passed the allocation.
+// Out of memory leaves no CUDA error behind: the caller may go on without.
 cudaError_t dev_malloc(void **p, size_t bytes, cudaStream_t s);
 template <typename T>
 cudaError_t dev_malloc(T **p, size_t bytes, cudaStream_t s)
