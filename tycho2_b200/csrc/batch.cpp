@@ -294,7 +294,7 @@ void Batch::fill_slot(int prec, const Member &m, BatchSlot &s) const
     s = BatchSlot();
     s.rec = v.rec;
     s.psi = v.psi;
-    s.iso = m.v[0].iso;
+    s.iso = v.iso;
     s.iso32 = prec ? v.iso32 : nullptr;
     s.sigma_s = v.sigs;
     s.scat = v.scat;
@@ -328,7 +328,7 @@ void Batch::fill_slot(int prec, const Member &m, BatchSlot &s) const
         s.active = 1;
         s.op = kOpSI;
         s.phi_in = m.cur;
-        s.q_fixed = m.v[0].qiso;
+        s.q_fixed = v.qiso;
         s.phi_out = m.nxt;
     } else if (prec == 0 && m.state == kRunOuter) {
         s.active = 1;
@@ -502,12 +502,26 @@ int Batch::pass(int prec, std::string &err)
         any = any || (prec == 0 ? m.state == kRunSI || m.state == kRunOuter
                                 : m.state == kRunInner || m.state == kRunFirst);
     if (!any) return kOk;
+    // a member swept on its own, or given another work order or cross sections,
+    // since the last pass: its records in this pass's order again, or (no room for
+    // the chain plan) the pass made anew in level form
+    if (graph_[prec] && ipw_[prec] == 0)
+        for (auto &m : members_) {
+            if (m.state == kDone || (prec == 1 && m.o.method != 2)) continue;
+            if (m.sw->compact_ready(prec, chain_form_[prec])) continue;
+            const int s = m.sw->device_view(prec, m.v[prec], err, true, chain_form_[prec]);
+            if (s == kErrOom && chain_form_[prec]) {
+                err.clear();
+                cudaGraphExecDestroy(graph_[prec]);
+                graph_[prec] = nullptr;
+                break;
+            }
+            TB_CHECK(s);
+        }
     // the graph (and with it the members' level shifts) before the slot table
     if (!graph_[prec]) TB_CHECK(build_graph(prec, err));
-    if (ipw_[prec] == 0)  // a member swept on its own since then
-        for (auto &m : members_)
-            if (m.state != kDone && (prec == 0 || m.o.method == 2) && !m.sw->compact_ready(prec, chain_form_[prec]))
-                TB_CHECK(m.sw->device_view(prec, m.v[prec], err, true, chain_form_[prec]));
+    for (auto &m : members_)
+        if (prec == 0 || m.o.method == 2) m.sw->fill_view(prec, ipw_[prec] == 0, m.v[prec]);
     for (size_t j = 0; j < n; ++j) fill_slot(prec, members_[j], h_slots_[prec][j]);
     cudaStream_t st = prec ? stream32_ : stream_;
     TB_CUDA(cudaMemcpyAsync(d_slots_[prec], h_slots_[prec], sizeof(BatchSlot) * n, cudaMemcpyHostToDevice, st));

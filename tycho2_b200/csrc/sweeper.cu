@@ -677,6 +677,12 @@ int Sweeper::device_view(int prec, DeviceView &v, std::string &err, bool compact
     TY_CUDA(cudaSetDevice(device_));
     TY_CHECK(ensure_records(prec, true, err, compact, chain));
     TY_CUDA(cudaStreamSynchronize(stream_));
+    fill_view(prec, compact, v);
+    return kOk;
+}
+
+void Sweeper::fill_view(int prec, bool compact, DeviceView &v) const
+{
     v.chain_off = chain_.off;
     v.rec = compact ? d_crec_[prec ? 1 : 0] : d_rec_[prec ? 1 : 0];
     v.psi = d_psi_;
@@ -692,7 +698,6 @@ int Sweeper::device_view(int prec, DeviceView &v, std::string &err, bool compact
     v.n_levels = sched_.n_levels;
     v.vg = record_vg(prec != 0, (uint32_t)G_);
     v.zero_row = prec ? 2 * zero_row_ : zero_row_;
-    return kOk;
 }
 
 // Allocates (once) and fills (once per cross-section set) the per-item

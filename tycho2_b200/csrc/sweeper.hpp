@@ -126,6 +126,10 @@ public:
     };
     // chain: the compact records in (direction, level) order.
     int device_view(int prec, DeviceView &v, std::string &err, bool compact, bool chain = false);
+    // The view as it stands now: buffers are released and made anew by later
+    // calls on the sweeper (work order, sources, scattering), so it is asked for
+    // again before each use.
+    void fill_view(int prec, bool compact, DeviceView &v) const;
     // Whether the compact records stand filled in that order.
     bool compact_ready(int prec, bool chain) const
     {
