@@ -131,11 +131,13 @@ int Batch::add(Sweeper *sw, const BatchOptions &o, int &id, std::string &err)
     Member m;
     m.sw = sw;
     m.o = o;
-    // the records in the order the passes will most likely sweep them in
-    const bool chain = !persist_ && sw->solver() == kSolveNoPivot;
-    TB_CHECK(member_view(sw, 0, m.v[0], chain && ipw_[0] == 0, err));
+    // compact records are filled when the form of the passes is known (build_graph)
+    auto view = [&](int prec) {
+        return ipw_[prec] ? sw->device_view(prec, m.v[prec], err, false) : sw->reserve_view(prec, m.v[prec], err, true);
+    };
+    TB_CHECK(view(0));
     if (o.method == 2) {
-        TB_CHECK(member_view(sw, 1, m.v[1], chain && ipw_[1] == 0, err));
+        TB_CHECK(view(1));
         const size_t n = sw->phi_size();
         TB_CUDA(dev_malloc(&m.r, sizeof(double) * n, stream_));
         TB_CUDA(dev_malloc(&m.d, sizeof(double) * n, stream_));
@@ -155,6 +157,19 @@ int Batch::add(Sweeper *sw, const BatchOptions &o, int &id, std::string &err)
     invalidate();
     return kOk;
 }
+
+double PassEstimate::add(const Sweeper &sw, int prec)
+{
+    const double G = (double)sw.n_groups();
+    const double tasks = (double)sw.n_cells() * G / record_vg(prec != 0, (uint32_t)sw.n_groups());
+    const double k = prec ? 0.0045 : G <= 2.0 ? 0.0052 : 0.0085;
+    const double chain = 1.1 * sw.schedule().n_levels + k * tasks;
+    longest_ = std::max(longest_, chain);
+    work_ += tasks * sw.n_angles();
+    return chain;
+}
+
+bool PassEstimate::chains(uint32_t levels) const { return longest_ <= std::max(2.7 * levels, work_ / 15e3); }
 
 // A member's device state with its records in chain order, or (no room for
 // the chain plan; build_graph then takes the level form) in level order.
@@ -377,28 +392,18 @@ int Batch::build_graph(int prec, std::string &err)
     for (const auto &m : members_) any_solver = any_solver || m.sw->solver() != kSolveNoPivot;
     block_[prec] = ipw == 0 && !persist_ && !any_solver;  // the level kernels keep FP32 rows as blocks then
     // As direction chains unless one direction of a large member would last
-    // longer than all levels as launches.  Measured on B200, us: a chain's
-    // level 1.1 + k per task (k: FP64 0.0052 with 1 or 2 groups, 0.0085 with
-    // more; FP32 0.0045); a level launch of the batch 2.7, and 15 tasks/ns.
-    // FP32 pass in ms, chains / launches: one 24^3 S8 G=8 member 1.43 / 1.69
-    // (estimates 1.02 / 1.42), one 24^3 S4 G=8 member 1.13 / 0.77 (1.02 / 0.68),
-    // 24 uneven members 1.92 / 2.32 (0.54 / 2.59).
+    // longer than all levels as launches (PassEstimate).
     std::vector<std::pair<double, uint32_t>> order;  // minus a chain's time, member
     std::vector<uint2> table;
-    double longest = 0.0, total = 0.0;
+    PassEstimate est;
     size_t n_chains = 0;
     for (uint32_t j = 0; j < n; ++j) {
         const Member &m = members_[j];
         if (prec == 1 && m.o.method != 2) continue;
-        const double G = (double)m.sw->n_groups(), tasks = (double)m.sw->n_cells() * G / m.v[prec].vg;
-        const double k = prec ? 0.0045 : G <= 2.0 ? 0.0052 : 0.0085, t = 1.1 * m.v[prec].n_levels + k * tasks;
-        order.emplace_back(-t, j);
-        longest = std::max(longest, t);
-        total += tasks * m.sw->n_angles();
+        order.emplace_back(-est.add(*m.sw, prec), j);
         n_chains += (size_t)m.sw->n_angles();
     }
-    const double launches = std::max(2.7 * max_levels_, total / 15e3);
-    bool chains = block_[prec] && longest <= launches && n_chains < (1ull << 31);
+    bool chains = block_[prec] && est.chains(max_levels_) && n_chains < (1ull << 31);
     // one block per SM up to three for each of the 148, else smaller ones: FP64
     // pass with 256 / 512 threads, 24 uneven members (2,088 chains) 2.52 / 2.75 ms,
     // 3 members (232 chains) 0.91 / 0.83

@@ -39,6 +39,22 @@ struct BatchMemberStats {
     int steps = 0;  // batch steps the member took part in
 };
 
+// Whether a pass sweeps as direction chains or level by level: the longest
+// chain against all levels as launches.  Measured on B200, us: a chain's
+// level 1.1 + k per task (k: FP64 0.0052 with 1 or 2 groups, 0.0085 with
+// more; FP32 0.0045); a level launch of the batch 2.7, and 15 tasks/ns.
+// FP32 pass in ms, chains / launches: one 24^3 S8 G=8 member 1.43 / 1.69
+// (estimates 1.02 / 1.42), one 24^3 S4 G=8 member 1.13 / 0.77 (1.02 / 0.68),
+// 24 uneven members 1.92 / 2.32 (0.54 / 2.59).
+class PassEstimate {
+public:
+    double add(const Sweeper &sw, int prec);  // one member; its chains' time, us
+    bool chains(uint32_t levels) const;       // levels: of the deepest member
+
+private:
+    double longest_ = 0.0, work_ = 0.0;
+};
+
 class Batch {
 public:
     ~Batch();

@@ -669,12 +669,21 @@ LevelArgs Sweeper::form_args(int prec, bool has_iso, const double *qang) const
     return p;
 }
 
-int Sweeper::device_view(int prec, DeviceView &v, std::string &err, bool compact, bool chain)
+int Sweeper::reserve_view(int prec, DeviceView &v, std::string &err, bool compact)
 {
     if (prec == 1 && !fp32_) { err = "sweeper was created without the FP32 sweep"; return kErrArg; }
     if (n_bound_) { err = "faces toward other partitions: not in a batch"; return kErrArg; }
     if (!have_xs_) { err = "cross sections not set"; return kErrMissing; }
     TY_CUDA(cudaSetDevice(device_));
+    TY_CHECK(reserve_records(prec, compact, err));
+    TY_CUDA(cudaStreamSynchronize(stream_));
+    fill_view(prec, compact, v);
+    return kOk;
+}
+
+int Sweeper::device_view(int prec, DeviceView &v, std::string &err, bool compact, bool chain)
+{
+    TY_CHECK(reserve_view(prec, v, err, compact));
     TY_CHECK(ensure_records(prec, true, err, compact, chain));
     TY_CUDA(cudaStreamSynchronize(stream_));
     fill_view(prec, compact, v);
@@ -700,32 +709,39 @@ void Sweeper::fill_view(int prec, bool compact, DeviceView &v) const
     v.zero_row = prec ? 2 * zero_row_ : zero_row_;
 }
 
-// Allocates (once) and fills (once per cross-section set) the per-item
-// records of the record variant for one precision.
+// Allocates (once) the per-item records of one precision.
+int Sweeper::reserve_records(int prec, bool compact, std::string &err)
+{
+    const int k = prec ? 1 : 0;
+    void *&buf = compact ? d_crec_[k] : d_rec_[k];
+    if (buf) return kOk;
+    const size_t bytes =
+        (compact ? compact_record_bytes(prec == 1) : record_bytes(prec == 1)) * sched_.n_padded;
+    cudaError_t e = dev_malloc(&buf, bytes, stream_);
+    if (e != cudaSuccess) {
+        buf = nullptr;
+        err = std::string(compact ? "compact records (" : "records (") + std::to_string(bytes >> 20) +
+              " MiB) do not fit: " + cudaGetErrorString(e);
+        return e == cudaErrorMemoryAllocation ? kErrOom : kErrCuda;
+    }
+    (compact ? crec_valid_[k] : rec_valid_[k]) = false;
+    return kOk;
+}
+
+// The same, filled (once per cross-section set) when these are known.
 int Sweeper::ensure_records(int prec, bool need_filled, std::string &err, bool compact, bool chain)
 {
     const int k = prec ? 1 : 0;
     if (chain) TY_CHECK(ensure_chain_plan(err));
+    TY_CHECK(reserve_records(prec, compact, err));
     if (compact && crec_chain_[k] != chain) {  // the same buffer in the other order
         crec_valid_[k] = false;
         crec_chain_[k] = chain;
     }
     void *&buf = compact ? d_crec_[k] : d_rec_[k];
     bool &valid = compact ? crec_valid_[k] : rec_valid_[k];
-    if (!buf) {
-        const size_t bytes =
-            (compact ? compact_record_bytes(prec == 1) : record_bytes(prec == 1)) * sched_.n_padded;
-        cudaError_t e = dev_malloc(&buf, bytes, stream_);
-        if (e != cudaSuccess) {
-            cudaGetLastError();
-            buf = nullptr;
-            err = std::string(compact ? "compact records (" : "records (") + std::to_string(bytes >> 20) +
-                  " MiB) do not fit: " + cudaGetErrorString(e);
-            return e == cudaErrorMemoryAllocation ? kErrOom : kErrCuda;
-        }
-        valid = false;
-    }
     if (!valid && have_xs_) {
+        TraceScope trace("sweeper.records");
         const LevelArgs p = level_args(prec, nullptr, nullptr, d_psi_);
         const uint64_t n = chain ? sched_.n_items : sched_.n_padded;
         const uint32_t *pos = chain ? chain_.pos : nullptr;

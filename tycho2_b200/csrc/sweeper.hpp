@@ -124,8 +124,13 @@ public:
         const uint32_t *chain_off;  // chain order: each direction's level offsets
         uint32_t n_levels, vg, zero_row;
     };
-    // chain: the compact records in (direction, level) order.
+    // The records are allocated; chain: the compact ones filled in (direction,
+    // level) order, else in level order.
     int device_view(int prec, DeviceView &v, std::string &err, bool compact, bool chain = false);
+    // The same without filling the records: whoever sweeps them knows the order.
+    int reserve_view(int prec, DeviceView &v, std::string &err, bool compact);
+    // The records of the sweeper's own form, allocated and filled.
+    int ensure_form_records(int prec, std::string &err);
     // The view as it stands now: buffers are released and made anew by later
     // calls on the sweeper (work order, sources, scattering), so it is asked for
     // again before each use.
@@ -232,6 +237,7 @@ private:
     // (and computes, when stale) its contents for the current cross sections.
     // chain: compact records in chain order.
     int ensure_records(int prec, bool need_filled, std::string &err, bool compact = false, bool chain = false);
+    int reserve_records(int prec, bool compact, std::string &err);
 
     std::shared_ptr<const MeshTables> tables_;
     Quadrature quad_;
@@ -300,8 +306,6 @@ private:
     // Direction chains (sweep_chains.cuh): made on first use.
     ChainPlan chain_;
     int ensure_chain_plan(std::string &err);
-    // The records of the form in use, allocated and filled.
-    int ensure_form_records(int prec, std::string &err);
     cudaError_t enqueue_chains(int prec, bool has_iso, const double *qang);
     // direct dataflow: a completion epoch per (item, group vector)
     uint32_t *d_flags_ = nullptr;
