@@ -523,7 +523,7 @@ def run_serve_leg(grp, dev, count, rates, seed=99):
                           "solves_per_s": grp.sum(len(done)) / grp.max(st_["makespan"]),
                           "build_p50_s": float(np.percentile([i["built"] - i["admitted"] for i in done], 50)),
                           "mean_in_batch": float(sum(i["finished"] - i["built"] for i in done) / span),
-                          "peak_in_batch": st_["peak_active"],
+                          "peak_in_batch": st_["peak_solving"],
                           "peak_resident_gb": st_["peak_bytes"] / 1e9, "batch_steps": st_["steps"]}
             big = [i for p, i in zip(params, info) if p["n"] == 48 and i["state"] == "done"]
             if big:  # where the large requests' latency goes

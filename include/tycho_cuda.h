@@ -597,8 +597,13 @@ int tycho_server_submit(tycho_server *s, const tycho_mesh *mesh, int sn_order, i
 /* Serves every submitted request; returns when all are done or failed. */
 int tycho_server_run(tycho_server *s);
 int tycho_server_request(const tycho_server *s, int id, tycho_request_info *info);
+/* Peak device bytes reserved; the most requests at once on the device, from
+   the start of their build (its uploads and record kernels run beside the
+   others' sweeps) to their result; batch steps; seconds until the last result. */
 int tycho_server_stats(const tycho_server *s, double *peak_bytes, int *peak_active, int *steps,
                        double *makespan);
+/* The most requests at once in the service's batches or with its solo solver. */
+int tycho_server_peak_solving(const tycho_server *s, int *peak_solving);
 
 #ifdef __cplusplus
 }

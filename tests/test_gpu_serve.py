@@ -100,3 +100,25 @@ def test_large_requests_solo_match_batched(built, method):
         else:
             assert rel_l1(ps, pb) <= 1e-8
             assert i_s["stats"]["sweeps_fp32"] > 0
+
+
+@pytest.mark.parametrize("large_items", [0.0, 1.0])
+def test_peak_solving_counts_batch_and_solo_only(built, large_items):
+    """Requests being built beside a solve count in peak_active, not in
+    peak_solving; requests that solve together (or queue for the solo solver)
+    count in both."""
+    import tycho2_b200 as ty
+    mesh = ty.TychoMesh.kuhn_cube(4, 0.05, 1, 1.0)
+    st, q = np.full(mesh.n_cells, 30.0), np.ones((mesh.n_cells, 4, 2))  # slow to converge: 1500 steps
+    bad = -st  # refused while the request is built
+    for second, solving in ((bad, 1), (st, 2)):
+        srv = ty.SolveServer(method="si", budget_bytes=8e9, setup_threads=2, err_max=1e-12, iter_max=1500,
+                             large_items=large_items or 1e9)
+        ids = [srv.submit(mesh, 4, 2, s, 0.9999 * st, None, q, arrival=0.0) for s in (st, second)]
+        srv.run()
+        stats = srv.stats()
+        assert srv.info(ids[0])["state"] == "done"
+        assert srv.info(ids[1])["state"] == ("failed" if second is bad else "done")
+        assert stats["peak_solving"] == solving
+        assert stats["peak_active"] >= solving
+        srv.close()

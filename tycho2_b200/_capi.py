@@ -140,6 +140,7 @@ SIGNATURES.update({
     "tycho_server_run": (C.c_int, [_P]),
     "tycho_server_request": (C.c_int, [_P, C.c_int, C.POINTER(RequestInfo)]),
     "tycho_server_stats": (C.c_int, [_P, _P, C.POINTER(C.c_int), C.POINTER(C.c_int), _P]),
+    "tycho_server_peak_solving": (C.c_int, [_P, C.POINTER(C.c_int)]),
 })
 
 _lib = None

@@ -898,4 +898,11 @@ int tycho_server_stats(const tycho_server *s, double *peak_bytes, int *peak_acti
     return TYCHO_OK;
 }
 
+int tycho_server_peak_solving(const tycho_server *s, int *peak_solving)
+{
+    if (!s || !peak_solving) return finish(TYCHO_ERR_ARG, "null server or result");
+    *peak_solving = s->s.peak_solving();
+    return TYCHO_OK;
+}
+
 }  // extern "C"

@@ -643,10 +643,14 @@ class SolveServer:
         return d
 
     def stats(self):
+        """peak_active: the most requests at once on the device, being built or
+        solved; peak_solving: of these, in the batches or with the solo solver."""
         pb, ms = C.c_double(), C.c_double()
-        pa, st = C.c_int(), C.c_int()
+        pa, st, ps = C.c_int(), C.c_int(), C.c_int()
         check(lib().tycho_server_stats(self._h, C.byref(pb), C.byref(pa), C.byref(st), C.byref(ms)))
-        return {"peak_bytes": pb.value, "peak_active": pa.value, "steps": st.value, "makespan": ms.value}
+        check(lib().tycho_server_peak_solving(self._h, C.byref(ps)))
+        return {"peak_bytes": pb.value, "peak_active": pa.value, "peak_solving": ps.value, "steps": st.value,
+                "makespan": ms.value}
 
     def close(self):
         if getattr(self, "_h", None) is not None and self._h.value and _capi._lib is not None:
