@@ -52,3 +52,33 @@ def test_default_form_equals_level_launches(built, n, sn, G, prec, chains):
     sw.apply(phi, out[2], prec)
     assert torch.equal(out[0].view(torch.int64), out[2].view(torch.int64))
     sw.close()
+
+
+@pytest.mark.parametrize("n,sn,G", [(13, 8, 2), (20, 8, 1), (20, 6, 2)])
+def test_chunked_sweep_on_chain_records(built, n, sn, G):
+    """Host sweeps of 64 MB and more go in chunks of directions, on the records of
+    the sweeper's own form: between applications by chains, and against the level
+    order of a configured sweeper, psi bit for bit."""
+    import torch
+    import tycho2_b200 as ty
+    mesh = ty.TychoMesh.kuhn_cube(n, 0.05, 5, 1.0)
+    sw = ty.SweeperCuda(mesh, sn, G)
+    assert sw.launches(0) == 3  # chains
+    rng = np.random.default_rng(n)
+    st = rng.lognormal(0.0, 0.5, mesh.n_cells)
+    sw.set_cross_sections(st, 0.4 * st)
+    src = rng.uniform(0.0, 1.0, sw.psi_shape)
+    assert src.nbytes >= 64 << 20
+    x = torch.tensor(rng.uniform(0.0, 1.0, sw.phi_shape), device="cuda")
+    y = [torch.empty_like(x) for _ in range(2)]
+    psi = [np.full(sw.psi_shape, np.nan) for _ in range(3)]
+    sw.apply(x, y[0])
+    sw.sweep(psi[0], src)
+    sw.apply(x, y[1])
+    sw.sweep(psi[1], src)
+    sw.configure(0, "levels", "compact", -96, 0, 2)
+    sw.sweep(psi[2], src)
+    assert torch.equal(y[0].view(torch.int64), y[1].view(torch.int64))
+    for other in psi[1:]:
+        assert np.array_equal(psi[0].view(np.uint64), other.view(np.uint64))
+    sw.close()

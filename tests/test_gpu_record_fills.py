@@ -54,6 +54,10 @@ CASES = {
     "batch by level launches": ("batch([sweeper(24, 4, 8)], 'mixed')", 2),
     "solved alone, then in a batch": ("s = sweeper(5, 4, 2); s.solve('mixed', iter_max=50, err_max=1e-8); "
                                       "batch([s], 'mixed')", 2),
+    "applied and swept in turn": ("s = sweeper(15, 8, 2, False)\n"  # 166 MB: swept in chunks
+                                  "from torch import zeros; x = zeros(s.phi_shape, dtype=float, device='cuda')\n"
+                                  "psi = np.empty(s.psi_shape)\n"
+                                  "for _ in range(3): s.apply(x, x.clone()); s.sweep(psi, psi * 0 + 1)", 1),
 }
 
 

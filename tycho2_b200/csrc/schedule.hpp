@@ -79,6 +79,10 @@ int build_schedule_device(const MeshTables &t, const Quadrature &q, Schedule &s,
 int angle_chunks_device(const uint32_t *d_items, uint64_t n_padded, const uint64_t *d_level_off, uint32_t n_levels,
                         uint32_t A, uint32_t K, uint32_t **d_pos, std::vector<uint64_t> &off, cudaStream_t st,
                         std::string &err);
+// pos[k], k < n_items: schedule positions in, their places in chain order out
+// (chain_pos: the schedule positions of all n_items items in that order).
+int chain_places_device(uint32_t *d_pos, const uint32_t *d_chain_pos, uint64_t n_items, uint64_t n_padded,
+                        cudaStream_t st, std::string &err);
 // s.tlevel from s.items and s.level_offset (every item of segment l has level l).
 void tlevel_from_items(Schedule &s, uint64_t n_cells, int n_angles);
 

@@ -144,6 +144,18 @@ __global__ void seg_starts_kernel(const uint32_t *__restrict__ keys, uint64_t n,
         for (uint32_t s = k + 1; s <= nseg; ++s) start[s] = n;
 }
 
+__global__ void invert_kernel(const uint32_t *__restrict__ pos, uint64_t n, uint32_t *__restrict__ place)
+{
+    const uint64_t k = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (k < n) place[pos[k]] = (uint32_t)k;
+}
+
+__global__ void look_up_kernel(const uint32_t *__restrict__ place, uint64_t n, uint32_t *__restrict__ pos)
+{
+    const uint64_t k = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (k < n) pos[k] = place[pos[k]];
+}
+
 // Key of schedule position i for the angle-chunked sweep: chunk(angle) *
 // n_levels + level(i), or the trailing bucket K * n_levels for padding.  The
 // level of position i is found by bisection of the level offsets.
@@ -403,6 +415,18 @@ int angle_chunks_device(const uint32_t *d_items, uint64_t n_padded, const uint64
     DevBuf &cur = vb.Current() == (uint32_t *)d_vals[0].p ? d_vals[0] : d_vals[1];
     *d_pos_out = (uint32_t *)cur.p;
     cur.p = nullptr;
+    return kOk;
+}
+
+int chain_places_device(uint32_t *d_pos, const uint32_t *d_chain_pos, uint64_t n_items, uint64_t n_padded,
+                        cudaStream_t st, std::string &err)
+{
+    DevBuf d_place;
+    TS_CUDA(take(d_place, sizeof(uint32_t) * n_padded, st));
+    invert_kernel<<<blocks_for(n_items), kThreads, 0, st>>>(d_chain_pos, n_items, (uint32_t *)d_place.p);
+    TS_CUDA(cudaGetLastError());
+    look_up_kernel<<<blocks_for(n_items), kThreads, 0, st>>>((const uint32_t *)d_place.p, n_items, d_pos);
+    TS_CUDA(cudaGetLastError());
     return kOk;
 }
 

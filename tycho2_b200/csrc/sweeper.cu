@@ -1151,8 +1151,13 @@ inline void stream_fence()
 
 int Sweeper::sweep_host_chunked(const double *source, double *psi, int K, std::string &err)
 {
-    TY_CHECK(ensure_records(0, true, err, true));  // kErrOom before any copy
-    if (chunk_k_ != K) {
+    // The records in the order of the sweeper's own form (chains or levels), so
+    // that they are not filled again at every change between apply and this call.
+    // kErrOom before any copy.
+    if (chains_[0].threads) TY_CHECK(ensure_form_records(0, err));
+    const bool chain = chains_[0].threads != 0;
+    if (!chain) TY_CHECK(ensure_records(0, true, err, true));
+    if (chunk_k_ != K || chunk_chain_ != chain) {
         for (auto &g : chunk_graphs_)
             if (g) cudaGraphExecDestroy(g);
         chunk_graphs_.clear();
@@ -1161,8 +1166,11 @@ int Sweeper::sweep_host_chunked(const double *source, double *psi, int K, std::s
         chunk_k_ = 0;
         TY_CHECK(angle_chunks_device(d_items_, sched_.n_padded, d_level_off_, sched_.n_levels, (uint32_t)A_,
                                      (uint32_t)K, &d_chunk_pos_, chunk_off_, stream_, err));
+        if (chain)
+            TY_CHECK(chain_places_device(d_chunk_pos_, chain_.pos, sched_.n_items, sched_.n_padded, stream_, err));
         chunk_graphs_.assign(K, nullptr);
         chunk_k_ = K;
+        chunk_chain_ = chain;
     }
     if (!h2d_stream_) TY_CUDA(cudaStreamCreateWithFlags(&h2d_stream_, cudaStreamNonBlocking));
     if (!d2h_stream_) TY_CUDA(cudaStreamCreateWithFlags(&d2h_stream_, cudaStreamNonBlocking));

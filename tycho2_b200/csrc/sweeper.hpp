@@ -315,6 +315,7 @@ private:
     // drop-in sweep in angle chunks: schedule positions grouped by chunk then
     // level, one level graph per chunk, copy streams and their events
     int chunk_k_ = 0;
+    bool chunk_chain_ = false;  // the positions are places in chain order
     uint32_t *d_chunk_pos_ = nullptr;
     std::vector<uint64_t> chunk_off_;
     std::vector<cudaGraphExec_t> chunk_graphs_;
