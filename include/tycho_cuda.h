@@ -543,7 +543,7 @@ int tycho_batch_timing(const tycho_batch *b, double *ms, int *passes, double *up
 /* Device bytes a resident request holds (upper estimate, before building).
    mixed != 0: the mixed-precision service (FP32 sweep state as well);
    compact != 0: the service's batch runs the direct kernels (ipw 0) on
-   compact records. */
+   compact records, in direction chains where they are faster. */
 uint64_t tycho_footprint_bytes(uint64_t n_cells, int sn_order, int n_groups, int mixed, int compact);
 
 /* Sweepers, batches and servers take device memory from one stream-ordered

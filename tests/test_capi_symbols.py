@@ -54,6 +54,19 @@ def test_footprint_estimate_covers_psi_and_records():
         assert ty.footprint_bytes(nc, sn, 2 * G, True, False) > b
 
 
+def test_footprint_estimate_lists_every_per_item_array():
+    """What grows with cells x directions, without the share for allocator
+    rounding: psi, face terms, item list and epochs, compact records, and the
+    chain plan with the sort that makes it (16 bytes an item at its peak)."""
+    import tycho2_b200 as ty
+    for nc, sn, G in [(1296, 4, 1), (82944, 8, 1), (82944, 8, 8), (663552, 8, 16)]:
+        items = nc * 2 * sn * sn
+        for mixed in (False, True):
+            listed = (ty.footprint_bytes(nc, sn, G, mixed, True) - (8 << 20)) * 32 / 33
+            per_item = 4 * G * 8 + 32 + 4 + 4 + 112 + 16 + ((16 + 64) if mixed else 0)
+            assert listed >= 1.05 * items * per_item  # 5 %: padding of the levels
+
+
 def test_header_is_plain_c(tmp_path):
     """The boundary is a C ABI: the header compiles as strict C99 (a cgo,
     JNI or ctypes binding sees no C++), and every struct zero-initialises."""
