@@ -75,3 +75,33 @@ def test_no_room_for_the_chain_plan(built, entry):
     if entry == "apply":
         assert sw.launches(0) > 3  # level launches, kept
     sw.close()
+
+
+def test_autotune_without_room_for_records(built):
+    """Shapes whose records do not fit are left out, the sweeper's own form among
+    them."""
+    import torch
+    import tycho2_b200 as ty
+    mesh = ty.TychoMesh.kuhn_cube(20, 0.05, 5, 1.0)  # 688 MB of FP64 compact records
+    rng = np.random.default_rng(3)
+    st = rng.lognormal(0.0, 0.5, mesh.n_cells)
+    q = rng.uniform(0.5, 1.0, (mesh.n_cells, 4, 1))
+    x = torch.tensor(q, device="cuda")
+    out = []
+    for low in (False, True):
+        sw = ty.SweeperCuda(mesh, 8, 1, **({"tpi64": 1} if low else {}))
+        sw.set_cross_sections(st, 0.4 * st)
+        sw.set_source(q, "isotropic")
+        ty.release_cached_memory(0)
+        blocks = fill_device(450 << 20) if low else []
+        try:
+            if low:
+                best = sw.autotune(0, reps=1)
+                assert best["variant"] in ("items", "tiles")
+            out.append(torch.empty_like(x))
+            sw.apply(x, out[-1])
+        finally:
+            del blocks
+            torch.cuda.empty_cache()
+        sw.close()
+    assert torch.equal(out[0].view(torch.int64), out[1].view(torch.int64))

@@ -555,9 +555,11 @@ int Sweeper::autotune(int prec, int reps, LaunchShape *best_shape, double *best_
     LaunchShape keep = shape_[prec ? 1 : 0];
     bool keep_default = false;
     // the default form first, then every launch shape
-    if (solver_ == kSolveNoPivot) {
+    int ds = kErrOom;
+    if (solver_ == kSolveNoPivot) ds = configure_default(prec, err);
+    if (ds != kErrOom) {  // else its records do not fit next to psi
         double ms[2];
-        TY_CHECK(configure_default(prec, err));
+        TY_CHECK(ds);
         TY_CHECK(time_sweeps(prec, 1, false, ms, err));
         TY_CHECK(time_sweeps(prec, reps, true, ms, err));
         best = ms[0];
