@@ -709,9 +709,9 @@ def run_b200(args):
     b64 = algorithmic_bytes(nc, A, G, info["n_incoming_interior"], 8)
     ach32 = b32 / (lvl32 * 1e-3) / 1e9
     ach64 = b64 / (lvl64 * 1e-3) / 1e9
-    own = args.shape == "default"
-    k32 = kernel_name(shape32, True, launches[1] if own else None)
-    k64 = kernel_name(shape64, False, launches[0] if own else None)
+    own32, own64 = shape32["knob"] == 0, shape64["knob"] == 0  # the sweeper's own form, also when autotuned
+    k32 = kernel_name(shape32, True, launches[1] if own32 else None)
+    k64 = kernel_name(shape64, False, launches[0] if own64 else None)
 
     # Solve-level check: mixed precision vs FP64 GMRES on the same problem.
     solve = None
@@ -812,8 +812,8 @@ def run_b200(args):
         parity = run_parity(args, dev, cpu, gpu_psi_hash, phi_c2, sample, large, serve)
 
     if rank == 0:
-        t32 = profiled_traffic(args.workload, traffic_family(shape32, True, own))
-        t64 = profiled_traffic(args.workload, traffic_family(shape64, False, own))
+        t32 = profiled_traffic(args.workload, traffic_family(shape32, True, own32))
+        t64 = profiled_traffic(args.workload, traffic_family(shape64, False, own64))
         line = {
             "metric": METRIC, "value": value, "unit": "updates/s", "n_gpus": world,
             "steps": args.steps, "warmup": warm, "ms_per_step": ms32,

@@ -318,10 +318,13 @@ int tycho_sweeper_levels(const tycho_sweeper *sw, uint32_t *tlevel, uint32_t *de
                   vector also -196 / -180 / -172: each upwind face's three
                   values summed once, in pairs of groups, 64 threads capped
                   at 102 / 85 / 73 registers),
-              4 = direct compact records: 64 B (FP32) / 96 B (FP64) per item
+              4 = direct compact records: 64 B (FP32) / 112 B (FP64) per item
                   holding the matrix inputs (face terms, sigma_t V/20, V/20)
                   and topology; the factors are rebuilt in registers with the
-                  same arithmetic; level schedule, knob as for 3;
+                  same arithmetic; level schedule, knob as for 3, or 0: the
+                  form a sweeper starts with (NoPivot: its own level kernels,
+                  or direction chains where levels are small), with its own
+                  vector width and streams;
      vector   records (2, 3): groups per vector access of a psi row (1, 2, or
               4 in FP32; must divide nGroups); 0 = the widest that divides
               nGroups (4 or 2 in FP32, 2 in FP64). */

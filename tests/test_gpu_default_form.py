@@ -82,3 +82,43 @@ def test_chunked_sweep_on_chain_records(built, n, sn, G):
     for other in psi[1:]:
         assert np.array_equal(psi[0].view(np.uint64), other.view(np.uint64))
     sw.close()
+
+
+@pytest.mark.parametrize("n,sn,G,solver", [(5, 4, 2, "NoPivot"), (20, 8, 7, "NoPivot"), (22, 8, 6, "NoPivot"),
+                                           (4, 4, 3, "CramerGlu")])
+def test_reported_shape_leads_back_to_the_default_form(built, n, sn, G, solver):
+    """shape() of a sweeper in its own form, given to configure() later, is that
+    form again: the same launches and the same bits."""
+    import torch
+    import tycho2_b200 as ty
+    mesh = ty.TychoMesh.kuhn_cube(n, 0.05, 5, 1.0)
+    sw = ty.SweeperCuda(mesh, sn, G, fp32=True, gauss_elim=solver)
+    rng = np.random.default_rng(n)
+    st = rng.lognormal(0.0, 0.5, mesh.n_cells)
+    sw.set_cross_sections(st, 0.4 * st)
+    x = torch.tensor(rng.uniform(0.0, 1.0, sw.phi_shape), device="cuda")
+    for prec in (0, 1):
+        kept, launches = sw.shape(prec), sw.launches(prec)
+        y = [torch.empty_like(x) for _ in range(2)]
+        sw.apply(x, y[0], prec)
+        for shape in [("compact", -172 if prec and G % 2 == 0 else -96, 0, 2)] * (solver == "NoPivot") + [("direct", 128)]:
+            sw.configure(prec, "levels", *shape)
+            assert sw.shape(prec) != kept  # nor is it the name of another one
+        sw.apply(x, y[1], prec)
+        sw.configure(prec, **kept)
+        assert sw.shape(prec) == kept and sw.launches(prec) == launches
+        sw.apply(x, y[1], prec)
+        assert torch.equal(y[0].view(torch.int64), y[1].view(torch.int64))
+    sw.close()
+
+
+def test_own_form_refuses_shapes_it_does_not_have(built):
+    import tycho2_b200 as ty
+    sw = ty.SweeperCuda(ty.TychoMesh.kuhn_cube(2, 0.05, 5, 1.0), 4, 4, fp32=True)
+    for prec, args in ((0, ("levels", "compact", 0, 1)), (1, ("levels", "compact", 0, 2)),
+                       (0, ("levels", "compact", 0, 0, 4)), (0, ("levels", "direct", 0)),
+                       (0, ("dataflow", "compact", 0))):
+        with pytest.raises(ty.TychoError) as e:
+            sw.configure(prec, *args)
+        assert e.value.status == 1, args
+    sw.close()

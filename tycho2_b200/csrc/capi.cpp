@@ -539,7 +539,7 @@ int tycho_sweeper_get_shape(const tycho_sweeper *h, int precision, tycho_launch_
 {
     if (!h || !shape || (precision != 0 && precision != 1))
         return finish(TYCHO_ERR_ARG, "bad sweeper, precision or shape");
-    const tycho::LaunchShape &sh = h->sw.shape(precision);
+    const tycho::LaunchShape sh = h->sw.shape(precision);
     shape->schedule = sh.schedule;
     shape->variant = sh.variant;
     shape->knob = sh.knob;

@@ -412,6 +412,13 @@ int Sweeper::configure(int prec, int schedule, int variant, int knob, std::strin
         return kErrArg;
     }
     if (vg == 0) vg = (int)record_vg(prec != 0, (uint32_t)G_);
+    if (schedule == 1 && variant == 4 && knob == 0) {
+        if (vg != (int)record_vg(prec != 0, (uint32_t)G_) || streams > 2) {
+            err = "the default form (compact, knob 0) takes its own vector width and streams";
+            return kErrArg;
+        }
+        return configure_default(prec, err);
+    }
     // one access moves up to 16 bytes (4 FP32 / 2 FP64 groups); the direct
     // variants on levels also take two such vectors per task (8 / 4)
     const bool halves = (prec == 1 && vg == 8) || (prec == 0 && vg == 4);
@@ -604,7 +611,7 @@ int Sweeper::autotune(int prec, int reps, LaunchShape *best_shape, double *best_
             }
     if (keep_default) TY_CHECK(configure_default(prec, err));
     else TY_CHECK(configure(prec, keep.schedule, keep.variant, keep.knob, err, keep.vg, keep.streams));
-    if (best_shape) *best_shape = shape_[prec ? 1 : 0];
+    if (best_shape) *best_shape = shape(prec);
     if (best_ms) *best_ms = best;
     return kOk;
 }

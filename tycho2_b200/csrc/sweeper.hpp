@@ -86,7 +86,13 @@ public:
     // the block kernel or, for small levels, in direction chains.
     int configure_default(int prec, std::string &err);
     int autotune(int prec, int reps, LaunchShape *best, double *best_ms, std::string &err);
-    const LaunchShape &shape(int prec) const { return shape_[prec ? 1 : 0]; }
+    // Knob 0: the default form of the compact variant.
+    LaunchShape shape(int prec) const
+    {
+        LaunchShape sh = shape_[prec ? 1 : 0];
+        if (block_[prec ? 1 : 0]) sh.knob = 0;
+        return sh;
+    }
     // Kernel launches of one operator application with the current shape
     // (source, the sweep's launches, psi -> phi).
     uint64_t launches_per_apply(int prec) const;

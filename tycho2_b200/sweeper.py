@@ -308,8 +308,9 @@ class SweeperCuda:
 
     def configure(self, precision, schedule, variant, knob, vector=0, streams=1):
         """schedule 'levels'|'dataflow'|'persist' (records only); variant 'items' (knob = lanes per item),
-        'tiles' (knob = warps per block), 'records' (knob = items per warp) or 'direct' (records
-        in registers, level schedule, knob = threads per block); vector = records' groups per
+        'tiles' (knob = warps per block), 'records' (knob = items per warp), 'direct' or 'compact' (records
+        in registers, level schedule, knob = threads per block; 'compact', 0 = the form a sweeper
+        starts with); vector = records' groups per
         psi-row access, 0 = widest dividing nGroups; streams: level schedule on 1, 2, 4 or 8 concurrent
         streams (octant groups)."""
         sh = _capi.LaunchShape(self.SCHEDULES[schedule], self.VARIANTS[variant], knob, vector, streams)
