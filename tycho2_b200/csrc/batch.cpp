@@ -404,10 +404,7 @@ int Batch::build_graph(int prec, std::string &err)
         n_chains += (size_t)m.sw->n_angles();
     }
     bool chains = block_[prec] && est.chains(max_levels_) && n_chains < (1ull << 31);
-    // one block per SM up to three for each of the 148, else smaller ones: FP64
-    // pass with 256 / 512 threads, 24 uneven members (2,088 chains) 2.52 / 2.75 ms,
-    // 3 members (232 chains) 0.91 / 0.83
-    chain_nt_[prec] = n_chains <= 3 * 148 ? 512 : 256;
+    chain_nt_[prec] = batch_chain_threads(n_chains);
     for (auto &m : members_)
         if (chains && (prec == 0 || m.o.method == 2)) {
             TB_CHECK(member_view(m.sw, prec, m.v[prec], true, err));

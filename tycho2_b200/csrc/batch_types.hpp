@@ -95,6 +95,8 @@ cudaError_t launch_batch_finish(const BatchSlot *slots, const BatchPlan &pl, uns
 template <typename Real>
 cudaError_t launch_batch_level(int ipw, const BatchSlot *slots, const BatchPlan &pl, uint32_t level,
                                const BatchCuts &cut, bool any_solver, cudaStream_t s);
+// Threads of a chain's block in a pass of so many chains.
+int batch_chain_threads(size_t n_chains);
 // The wavefront of a pass as direction chains (compact records in chain
 // order, NoPivot): n blocks of nt
 // (256 or 512) threads, one per (slot, direction) of the table.

@@ -462,8 +462,8 @@ static cudaError_t launch_phi(const Real *psi, const double *w, double *phi, uin
 {
     // tiles of 256 elements; fewer cells a tile where those would not give
     // every SM four blocks (8^3 of 4 elements: 512 tiles of 6 cells, not 48 of 64)
-    constexpr uint64_t kBlocks = 592;
-    const uint64_t even = (nc + kBlocks - 1) / kBlocks;
+    const uint64_t blocks = 4 * (uint64_t)std::max(device_sm_count(), 1);
+    const uint64_t even = (nc + blocks - 1) / blocks;
     const PhiPlan plan = phi_plan<Form>((uint32_t)std::min<uint64_t>(kPhiTile / (4 * Gp), even),
                                         4 * Gp * (uint32_t)sizeof(Real), A);
     const unsigned grid = (unsigned)((nc + plan.cells - 1) / plan.cells);

@@ -958,7 +958,6 @@ int Sweeper::levels(int prec, bool has_iso, const double *qang, cudaEvent_t beg,
 // dependent launch.
 cudaError_t Sweeper::enqueue_levels(int prec, bool has_iso, const double *qang)
 {
-    if (chains_[prec ? 1 : 0].threads) return enqueue_chains(prec, has_iso, qang);
     const LaunchShape &sh = shape_[prec ? 1 : 0];
     const LevelArgs p = form_args(prec, has_iso, qang);
     cudaError_t le = cudaSuccess;
