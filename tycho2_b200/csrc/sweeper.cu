@@ -685,7 +685,6 @@ int Sweeper::reserve_view(int prec, DeviceView &v, std::string &err, bool compac
     if (!have_xs_) { err = "cross sections not set"; return kErrMissing; }
     TY_CUDA(cudaSetDevice(device_));
     TY_CHECK(reserve_records(prec, compact, err));
-    TY_CUDA(cudaStreamSynchronize(stream_));
     fill_view(prec, compact, v);
     return kOk;
 }

@@ -133,7 +133,8 @@ public:
     // The records are allocated; chain: the compact ones filled in (direction,
     // level) order, else in level order.
     int device_view(int prec, DeviceView &v, std::string &err, bool compact, bool chain = false);
-    // The same without filling the records: whoever sweeps them knows the order.
+    // The same without filling the records or waiting: whoever sweeps them knows
+    // the order, and asks for device_view before.
     int reserve_view(int prec, DeviceView &v, std::string &err, bool compact);
     // The records of the sweeper's own form, allocated and filled.
     int ensure_form_records(int prec, std::string &err);
