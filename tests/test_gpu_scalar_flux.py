@@ -56,3 +56,25 @@ def test_batched_scalar_flux(built):
         b.close()
     for sw in sweepers:
         sw.close()
+
+
+@pytest.mark.parametrize("members", [[(18, 2, 8), (3, 4, 3)], [(24, 2, 16), (21, 2, 33), (5, 4, 1)],
+                                     [(20, 2, 7), (22, 4, 1)]])
+def test_batched_streaming_passes_of_larger_members(built, members):
+    """Sums of chunks (4096 elements of phi) for which the streaming passes take a
+    chunk whole and in quarters, and several tiles of cells one after the other:
+    phi of the single solver's source iteration bit for bit, the mixed solve's to its
+    tolerance (1e-9 of a sum; 1e-7 allowed of each element)."""
+    import tycho2_b200 as ty
+    sweepers = [make(n, sn, G, True) for n, sn, G in members]
+    for method, tol in (("si", 0.0), ("mixed", 1e-7)):
+        b = ty.BatchSolver()
+        ids = [b.add(sw, method, err_max=1e-10 if method == "si" else 1e-9) for sw in sweepers]
+        b.run()
+        for sw, i in zip(sweepers, ids):
+            phi = b.result(i)[0]
+            want = sw.solve("si", err_max=1e-10, want_psi=False)[0]
+            assert np.abs(phi / want - 1.0).max() <= tol
+        b.close()
+    for sw in sweepers:
+        sw.close()

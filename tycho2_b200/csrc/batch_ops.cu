@@ -9,22 +9,42 @@ namespace {
 
 // Grid-stride loop over the active members' phi chunks: fn(slot, first
 // element, end element, chunk index).
-// PARTS > 1: each chunk in that many parts, one block iteration per part.
-template <uint32_t PARTS = 1, typename Fn>
-__device__ __forceinline__ void for_each_chunk(const BatchSlot *__restrict__ slots, const BatchPlan &pl, Fn fn)
+// parts(chunks): how many parts each chunk is taken in, one block iteration
+// per part (a power of two).
+template <typename Parts, typename Fn>
+__device__ __forceinline__ void for_each_part(const BatchSlot *__restrict__ slots, const BatchPlan &pl, Parts parts,
+                                              Fn fn)
 {
-    constexpr uint32_t part = kBatchChunk / PARTS;
     const uint32_t n_act = *pl.n_act;
-    const uint32_t total = pl.chunk_prefix[n_act] * PARTS;
+    const uint32_t P = parts(pl.chunk_prefix[n_act]), part = kBatchChunk / P;
+    const uint32_t total = pl.chunk_prefix[n_act] * P;
     for (uint32_t bp = blockIdx.x; bp < total; bp += gridDim.x) {
-        const uint32_t b = bp / PARTS;
+        const uint32_t b = bp / P;
         const uint32_t k = upper_index(n_act, b, [&](uint32_t m) { return pl.chunk_prefix[m]; });
         const BatchSlot &s = slots[pl.act[k]];
         const uint64_t n = s.nc * 4 * s.G;
-        const uint64_t i0 = (uint64_t)(b - pl.chunk_prefix[k]) * kBatchChunk + bp % PARTS * part;
+        const uint64_t i0 = (uint64_t)(b - pl.chunk_prefix[k]) * kBatchChunk + bp % P * part;
         const uint64_t i1 = i0 + part < n ? i0 + part : n;
         fn(s, i0, i1, b);
     }
+}
+
+template <typename Fn>
+__device__ __forceinline__ void for_each_chunk(const BatchSlot *__restrict__ slots, const BatchPlan &pl, Fn fn)
+{
+    for_each_part(slots, pl, [](uint32_t) { return 1u; }, fn);
+}
+
+// The parts for a streaming pass over so many chunks: whole ones where each
+// block has one, else quarters (256 (cell, group) pairs, one per thread) down to
+// a quarter of that, and 256 elements for the few that are left.  With 256
+// elements always, three quarters of the scatter's threads had no pair: 25
+// members of G=8 484 us a pass, with this rule 162; 256 uneven members FP64
+// 61.0 -> 59.4 ms, one 24^3 S4 G=8 member FP32 0.821 -> 0.778; five members of at
+// most 12^3 cells as before (0.450).
+__device__ __forceinline__ uint32_t stream_parts(uint32_t chunks)
+{
+    return chunks >= gridDim.x ? 1u : chunks * 4u >= gridDim.x ? 4u : 16u;
 }
 
 __global__ void __launch_bounds__(256) batch_accept_kernel(const BatchSlot *__restrict__ slots, BatchPlan pl)
@@ -40,7 +60,7 @@ __global__ void __launch_bounds__(256) batch_accept_kernel(const BatchSlot *__re
 // per element.  Bit-identical either way.
 __global__ void __launch_bounds__(256) batch_scatter_kernel(const BatchSlot *__restrict__ slots, BatchPlan pl)
 {
-    for_each_chunk<kBatchChunk / 256>(slots, pl, [&](const BatchSlot &s, uint64_t i0, uint64_t i1, uint32_t) {
+    for_each_part(slots, pl, stream_parts, [&](const BatchSlot &s, uint64_t i0, uint64_t i1, uint32_t) {
         const uint32_t row = 4u * s.G;
         if (i0 >= i1) return;
         if (256 % row == 0) {
@@ -86,7 +106,7 @@ __global__ void __launch_bounds__(PhiBatch::kThreads)
 batch_psi_to_phi_kernel(const BatchSlot *__restrict__ slots, BatchPlan pl)
 {
     extern __shared__ __align__(16) unsigned char stages[];
-    for_each_chunk<kBatchChunk / kPhiTile>(slots, pl, [&](const BatchSlot &s, uint64_t i0, uint64_t i1, uint32_t) {
+    for_each_part(slots, pl, [](uint32_t) { return kBatchChunk / kPhiTile; }, [&](const BatchSlot &s, uint64_t i0, uint64_t i1, uint32_t) {
         if (i0 >= i1) return;
         const uint32_t row = 4 * s.G;
         const uint64_t c0 = (i0 + row - 1) / row;
