@@ -92,13 +92,16 @@ __global__ void __launch_bounds__(256) batch_scatter_kernel(const BatchSlot *__r
     });
 }
 
-// The cells that start in 256 elements of a chunk per block iteration, so even
-// a few small members fill the GPU: whole chunks per block took 252 us for
-// five members of at most 12^3 cells, whose sweep takes 143.  At most 255
-// elements and a row (256) of them, two per thread.  Streamed through
-// shared-memory stages: 24 members of at most 24^3 cells, FP64 529 -> 336 us a
-// pass, FP32 349 -> 255 (with 3 stages of 8 KB 512 and 462, with 3 of 12 KB
-// 353 and 284); five members of at most 12^3 cells 51 -> 30.
+// The cells that start in a part of a chunk (stream_parts) per block iteration,
+// in tiles of about 256 elements (at most 255 and a row), two per thread: whole
+// chunks per block took 252 us for five members of at most 12^3 cells, whose
+// sweep takes 143.  Streamed through shared-memory stages: 24 members of at most
+// 24^3 cells, FP64 529 -> 336 us a pass, FP32 349 -> 255 (with 3 stages of 8 KB 512
+// and 462, with 3 of 12 KB 353 and 284); five members of at most 12^3 cells 51 ->
+// 30.  The stages of a part's tiles are one sequence: drained at every tile, a
+// tile of few directions waited for its loads (two 24^3 S2 G=16 members FP32 236
+// us, one 24^3 S4 G=8 111, by loads into registers 107 and 88); a pass of those
+// 1.24 -> 1.10 and 0.778 -> 0.763 ms, of 256 uneven members FP64 59.4 -> 58.1.
 struct PhiBatch { static constexpr int kElems = 2, kThreads = 256, kStages = 4, kBytes = 12288; };
 
 template <typename Real>
@@ -106,25 +109,25 @@ __global__ void __launch_bounds__(PhiBatch::kThreads)
 batch_psi_to_phi_kernel(const BatchSlot *__restrict__ slots, BatchPlan pl)
 {
     extern __shared__ __align__(16) unsigned char stages[];
-    for_each_part(slots, pl, [](uint32_t) { return kBatchChunk / kPhiTile; }, [&](const BatchSlot &s, uint64_t i0, uint64_t i1, uint32_t) {
+    for_each_part(slots, pl, stream_parts, [&](const BatchSlot &s, uint64_t i0, uint64_t i1, uint32_t) {
         if (i0 >= i1) return;
         const uint32_t row = 4 * s.G;
         const uint64_t c0 = (i0 + row - 1) / row;
         const uint32_t n = (uint32_t)((i1 + row - 1) / row - c0);
         if (n == 0) return;
         const PhiPlan plan = phi_plan<PhiBatch>((kPhiTile + row - 1) / row, row * (uint32_t)sizeof(Real), s.A);
-        double v[2];
-        phi_of_tile<Real, PhiBatch>((const Real *)s.psi + c0 * s.A * row, s.w, n, s.A, row, plan, stages, v);
-        const uint32_t e = 2 * threadIdx.x;
-        const uint64_t i = c0 * row + e;
-        if (e < n * row) {
+        phi_of_tiles<Real, PhiBatch>((const Real *)s.psi + c0 * s.A * row, s.w, n, s.A, row, plan, stages,
+                                     [&](uint32_t t0, uint32_t tn, const double (&v)[2]) {
+            const uint32_t e = 2 * threadIdx.x;
+            const uint64_t i = (c0 + t0) * row + e;
+            if (e >= tn * row) return;
             if (s.blk) {
                 s.phi_out[block_to_plain(i, s.G, s.blk)] = v[0];
                 s.phi_out[block_to_plain(i + 1, s.G, s.blk)] = v[1];
             } else {
                 *reinterpret_cast<double2 *>(s.phi_out + i) = make_double2(v[0], v[1]);
             }
-        }
+        });
         __syncthreads();  // the stages are free for the next
     });
 }

@@ -81,21 +81,22 @@ psi_to_phi_kernel(const Real *__restrict__ psi, const double *__restrict__ w, do
     pdl_wait_prerequisites();
     const uint64_t c0 = (uint64_t)blockIdx.x * plan.cells;
     const uint32_t row = 4 * Gp, n = (uint32_t)min((uint64_t)plan.cells, nc - c0);
-    double s[Form::kElems];
-    phi_of_tile<Real, Form>(psi + c0 * A * row, w, n, A, row, plan, stages, s);
+    phi_of_tiles<Real, Form>(psi + c0 * A * row, w, n, A, row, plan, stages,
+                             [&](uint32_t, uint32_t, const double (&s)[Form::kElems]) {
 #pragma unroll
-    for (int k = 0; k < Form::kElems; ++k) {
-        const uint32_t e = Form::kElems * threadIdx.x + k;
-        if (e >= n * row) return;
-        const uint32_t cl = e / row, q = e - cl * row;
-        uint32_t v = q / G, g = q - v * G;
-        if (blk) {
-            const uint32_t b = q / (4 * blk), r = q - b * 4 * blk;
-            v = r / blk;
-            g = b * blk + (r - v * blk);
+        for (int k = 0; k < Form::kElems; ++k) {
+            const uint32_t e = Form::kElems * threadIdx.x + k;
+            if (e >= n * row) return;
+            const uint32_t cl = e / row, q = e - cl * row;
+            uint32_t v = q / G, g = q - v * G;
+            if (blk) {
+                const uint32_t b = q / (4 * blk), r = q - b * 4 * blk;
+                v = r / blk;
+                g = b * blk + (r - v * blk);
+            }
+            if (g < G) phi[(c0 + cl) * 4 * G + v * G + g] = s[k];
         }
-        if (g < G) phi[(c0 + cl) * 4 * G + v * G + g] = s[k];
-    }
+    });
 }
 
 // One thread per (cell, group): the group's four vertex elements (groups

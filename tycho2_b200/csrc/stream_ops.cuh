@@ -146,49 +146,67 @@ __host__ __device__ inline PhiPlan phi_plan(uint32_t cells, uint32_t row_bytes, 
     return p;
 }
 
-// The thread's elements of n cells (n <= p.cells) from `psi` on, rows of `row`
-// values: threads beyond n * row elements return garbage.  smem: the stages,
-// each p.cells * p.stride bytes, 16-byte aligned.  All threads of a block of
-// Form::kThreads must call it.
-template <typename Real, typename Form>
-__device__ __forceinline__ void phi_of_tile(const Real *__restrict__ psi, const double *__restrict__ w, uint32_t n,
-                                            uint32_t A, uint32_t row, const PhiPlan &p, unsigned char *smem,
-                                            double (&s)[Form::kElems])
+// The elements of n cells from `psi` on, rows of `row` values, in tiles of
+// p.cells: emit(first cell of the tile, its cells, s) with the thread's elements
+// E * threadIdx.x ... of the tile's (garbage beyond its end).  The stages of all
+// tiles are one sequence, so a tile's first ones are on their way while the tile
+// before is summed.  smem: the stages, each p.cells * p.stride bytes, 16-byte
+// aligned.  All threads of a block of Form::kThreads must call it.
+template <typename Real, typename Form, typename Emit>
+__device__ __forceinline__ void phi_of_tiles(const Real *__restrict__ psi, const double *__restrict__ w, uint32_t n,
+                                             uint32_t A, uint32_t row, const PhiPlan &p, unsigned char *smem, Emit emit)
 {
     constexpr int E = Form::kElems, NS = Form::kStages;
     struct alignas(E * sizeof(Real)) Vec { Real x[E]; };
     const uint32_t rb = row * (uint32_t)sizeof(Real), cell = threadIdx.x >> p.shift;
-    const uint32_t lane = threadIdx.x & ((1u << p.shift) - 1u), stages = (A + p.angles - 1) / p.angles;
+    const uint32_t lane = threadIdx.x & ((1u << p.shift) - 1u);
     const uint32_t stage_bytes = p.cells * p.stride;
+    const size_t tile_bytes = (size_t)p.cells * A * rb;
     const unsigned char *src = reinterpret_cast<const unsigned char *>(psi) + (size_t)cell * A * rb;
-    auto load = [&](uint32_t st) {
-        if (st < stages && cell < n) {
-            const uint32_t a0 = st * p.angles, bytes = min(p.angles, A - a0) * rb;
-            unsigned char *d = smem + (st % NS) * stage_bytes + cell * p.stride;
-            const unsigned char *q = src + (size_t)a0 * rb;
-            for (uint32_t x = lane * 16; x < bytes; x += 16u << p.shift) cp_async16(d + x, q + x);
+    uint32_t ld_c0 = 0, ld_a0 = 0, ld_slot = 0;  // the next stage to load: its tile's first cell, first angle, place
+    auto load = [&] {
+        if (ld_c0 < n) {
+            if (cell < p.cells && ld_c0 + cell < n) {
+                const uint32_t bytes = min(p.angles, A - ld_a0) * rb;
+                unsigned char *d = smem + ld_slot * stage_bytes + cell * p.stride;
+                const unsigned char *q = src + (size_t)ld_a0 * rb;
+                for (uint32_t x = lane * 16; x < bytes; x += 16u << p.shift) cp_async16(d + x, q + x);
+            }
+            ld_slot = ld_slot + 1 == NS ? 0 : ld_slot + 1;
+            ld_a0 += p.angles;
+            if (ld_a0 >= A) {
+                ld_a0 = 0;
+                ld_c0 += p.cells;
+                src += tile_bytes;
+            }
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
 #pragma unroll
-    for (uint32_t st = 0; st < NS - 1; ++st) load(st);
-    const uint32_t e = E * threadIdx.x < n * row ? E * threadIdx.x : 0, ec = e / row;
+    for (int k = 0; k < NS - 1; ++k) load();
+    const uint32_t e = E * threadIdx.x < p.cells * row ? E * threadIdx.x : 0, ec = e / row;
     const unsigned char *mine = smem + ec * p.stride + (e - ec * row) * sizeof(Real);
+    uint32_t slot = 0;
+    for (uint32_t c0 = 0; c0 < n; c0 += p.cells) {
+        double s[E];
 #pragma unroll
-    for (int k = 0; k < E; ++k) s[k] = 0.0;
-    for (uint32_t st = 0; st < stages; ++st) {
-        asm volatile("cp.async.wait_group %0;" ::"n"(NS - 2) : "memory");
-        __syncthreads();      // stage st is there; all threads are done with st - 1
-        load(st + NS - 1);    // into the latter's place
-        const uint32_t a0 = st * p.angles, na = min(p.angles, A - a0);
-        const unsigned char *q = mine + (st % NS) * stage_bytes;
+        for (int k = 0; k < E; ++k) s[k] = 0.0;
+        for (uint32_t a0 = 0; a0 < A; a0 += p.angles) {
+            asm volatile("cp.async.wait_group %0;" ::"n"(NS - 2) : "memory");
+            __syncthreads();  // the stage is there; all threads are done with the one before
+            load();           // into the latter's place
+            const uint32_t na = min(p.angles, A - a0);
+            const unsigned char *q = mine + slot * stage_bytes;
+            slot = slot + 1 == NS ? 0 : slot + 1;
 #pragma unroll 4
-        for (uint32_t a = 0; a < na; ++a, q += rb) {
-            const Vec v = *reinterpret_cast<const Vec *>(q);
-            const double wa = w[a0 + a];
+            for (uint32_t a = 0; a < na; ++a, q += rb) {
+                const Vec v = *reinterpret_cast<const Vec *>(q);
+                const double wa = w[a0 + a];
 #pragma unroll
-            for (int k = 0; k < E; ++k) s[k] += (double)v.x[k] * wa;
+                for (int k = 0; k < E; ++k) s[k] += (double)v.x[k] * wa;
+            }
         }
+        emit(c0, min(p.cells, n - c0), s);
     }
 }
 
