@@ -15,6 +15,8 @@ BATCHES = {
     "chains-256": [(6, 8, 1), (5, 8, 8), (7, 8, 6), (4, 8, 5), (1, 4, 2)],
     "levels-fp64": [(15, 2, 8), (3, 2, 1), (4, 2, 2), (5, 2, 3)],
     "levels-both": [(21, 2, 16), (3, 2, 1), (4, 2, 2), (5, 2, 5)],
+    "levels-direct": [(21, 2, 16), (9, 2, 12), (4, 2, 20)],            # every row plain
+    "levels-many-rows": [(21, 2, 16), (5, 2, 8), (4, 2, 4), (3, 2, 7), (6, 2, 6), (2, 2, 64)],
 }
 
 

@@ -324,7 +324,8 @@ void Batch::fill_slot(int prec, const Member &m, BatchSlot &s) const
     s.level_shift = m.shift;
     s.solver = (uint32_t)m.sw->solver();
     s.zero_row = v.zero_row;
-    s.blk = prec && block_[prec] ? block_width(s.G) : 0u;
+    s.direct = block_[prec] && !chain_form_[prec] && level_direct(prec != 0, s.G);
+    s.blk = prec && block_[prec] && !s.direct ? block_width(s.G) : 0u;
     s.chain_off = v.chain_off;
     // levels of so few tasks by halves of the block in turn (10 members up to
     // 10^3, 256 threads: FP64 pass 199 -> 181 us; 5 members up to 16^3, 512 threads:
@@ -371,26 +372,27 @@ int Batch::build_graph(int prec, std::string &err)
     if (!graph_[0] && !graph_[1]) assign_shifts();  // the member set changed
     const int ipw = ipw_[prec];
     const uint32_t n = (uint32_t)members_.size();
+    bool any_solver = false;
+    for (const auto &m : members_) any_solver = any_solver || m.sw->solver() != kSolveNoPivot;
+    block_[prec] = ipw == 0 && !persist_ && !any_solver;  // the level kernels keep FP32 rows as blocks then
     // Blocks per level and class: enough for every member's chunks at once
     // (fewer when some are idle; the kernel's warps then exit at once).
     std::vector<BatchCuts> cuts(max_levels_);
     for (uint32_t L = 0; L < max_levels_; ++L) {
-        uint64_t chunks[kBatchClasses] = {0, 0, 0};
+        uint64_t chunks[kBatchClasses] = {};
         for (const auto &m : members_) {
             const auto &lo = m.sw->schedule().level_offset;
             if (L < m.shift || L - m.shift >= m.v[0].n_levels) continue;
             const uint64_t items = lo[L - m.shift + 1] - lo[L - m.shift];
             const uint32_t vg = m.v[prec].vg;
-            chunks[vg == 4 ? 2 : vg == 2 ? 1 : 0] +=
+            const bool direct = block_[prec] && level_direct(prec != 0, (uint32_t)m.sw->n_groups());
+            chunks[direct ? kDirectClass : vg == 4 ? 2 : vg == 2 ? 1 : 0] +=
                 ipw ? items / ipw : items / 32 * ((uint64_t)m.sw->n_groups() / vg);
         }
         cuts[L].c[0] = 0;
         for (uint32_t c = 0; c < kBatchClasses; ++c)
             cuts[L].c[c + 1] = cuts[L].c[c] + (unsigned)std::min<uint64_t>((chunks[c] + 3) / 4, kLevelGridCap);
     }
-    bool any_solver = false;
-    for (const auto &m : members_) any_solver = any_solver || m.sw->solver() != kSolveNoPivot;
-    block_[prec] = ipw == 0 && !persist_ && !any_solver;  // the level kernels keep FP32 rows as blocks then
     // As direction chains unless one direction of a large member would last
     // longer than all levels as launches (PassEstimate).
     std::vector<std::pair<double, uint32_t>> order;  // minus a chain's time, member

@@ -12,8 +12,7 @@ cudaError_t launch_batch_level<float>(int ipw, const BatchSlot *slots, const Bat
                                       const BatchCuts &cut, bool any_solver, cudaStream_t s)
 {
     const void *fn = ipw == 0    ? (any_solver ? (const void *)batch_direct_level_kernel<float, true>
-                                               : batch_deep(cut) ? (const void *)batch_direct_level_kernel<float, false, 5>
-                                                 : (const void *)batch_direct_level_kernel<float, false, 4, false>)
+                                               : batch_level_fn<float>(cut))
                      : ipw == 8  ? (const void *)batch_level_kernel<float, 8>
                      : ipw == 16 ? (const void *)batch_level_kernel<float, 16>
                      : ipw == 32 ? (const void *)batch_level_kernel<float, 32>

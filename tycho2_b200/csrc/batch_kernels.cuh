@@ -32,7 +32,10 @@ namespace tycho {
 
 constexpr int kBatchPlanThreads = 256;
 
-__host__ __device__ __forceinline__ uint32_t batch_class(uint32_t vg) { return vg == 4 ? 2u : vg == 2 ? 1u : 0u; }
+__device__ __forceinline__ uint32_t batch_class(const BatchSlot &s)
+{
+    return s.direct ? kDirectClass : s.vg == 4 ? 2u : s.vg == 2 ? 1u : 0u;
+}
 
 __device__ __forceinline__ uint32_t block_exclusive_scan(uint32_t v, uint32_t *total)
 {
@@ -80,7 +83,7 @@ batch_plan_kernel(const BatchSlot *__restrict__ slots, uint32_t n_slots, uint32_
                 uint64_t lo = 0;
                 const uint32_t sh = j < n_slots ? slots[j].level_shift : 0u;
                 if (j < n_slots && slots[j].active && L >= sh && L - sh < slots[j].n_levels &&
-                    batch_class(slots[j].vg) == cls) {
+                    batch_class(slots[j]) == cls) {
                     lo = slots[j].level_off[L - sh];
                     const uint64_t items = slots[j].level_off[L - sh + 1] - lo;
                     // IPW items per chunk; IPW == 0 (direct kernel): 32 (item, group vector) tasks
@@ -207,9 +210,9 @@ constexpr uint32_t kBatchSegSmem = 256, kBatchSegWhole = 32;
 // One chunk (32 tasks of one member at one level) of the direct form: the
 // member's segment found by binary search, its compact record rebuilt in
 // registers, the source loaded, then (after `wait`, which the caller uses to
-// wait for the previous level) the upwind rows (read as MODE says) and the
-// solve.
-template <typename Real, int VG, bool ANY, int MODE, typename Wait>
+// wait for the previous level) the upwind rows (read as MODE says; ALL: of the
+// four faces at once) and the solve.
+template <typename Real, int VG, bool ANY, int MODE, bool ALL, typename Wait>
 __device__ __forceinline__ void batch_direct_chunk(const BatchSeg *segs, uint32_t nseg, uint32_t ch, uint32_t lane,
                                                    Wait wait)
 {
@@ -247,7 +250,7 @@ __device__ __forceinline__ void batch_direct_chunk(const BatchSeg *segs, uint32_
 #pragma unroll
                 for (int e = 0; e < VG; ++e) q[v][e] = in.q[v][e];
         };
-        sweep_task<Real, VG, MODE, true, false, false>(p, R, g, source);
+        sweep_task<Real, VG, MODE, true, ALL, false>(p, R, g, source);
     }
 }
 
@@ -310,7 +313,8 @@ __device__ __forceinline__ const BatchSeg *batch_stage_segs(const BatchPlan &pl,
 // only the first chunks (up to kBatchSegSmem, beyond that they are searched in
 // global memory), and the segment found is read from global memory, where the
 // blocks of an SM share it in L1.
-template <typename Real, int VG, bool ANY, bool DEEP>
+// DIRECT: the members of class kDirectClass.
+template <typename Real, int VG, bool ANY, bool DEEP, bool DIRECT>
 __device__ __forceinline__ void batch_level_body(const BatchPlan &pl, uint32_t L, uint32_t cls, uint32_t blk,
                                                  uint32_t nblk, BatchSeg *sseg, RecordStage<Real> &S, bool &waited)
 {
@@ -337,7 +341,7 @@ __device__ __forceinline__ void batch_level_body(const BatchPlan &pl, uint32_t L
         const BatchSeg &sg =
             whole ? sseg[upper_index(nseg, ch, [&](uint32_t m) { return sseg[m].chunk_begin; })]
                   : segs[upper_index(nseg, ch, [&](uint32_t m) { return begin[m]; })];
-        if constexpr (ANY) batch_direct_chunk<Real, VG, true, kLoadPlain>(&sg, 1, ch, lane, wait);
+        if constexpr (ANY || DIRECT) batch_direct_chunk<Real, VG, ANY, kLoadPlain, true>(&sg, 1, ch, lane, wait);
         else if (sizeof(Real) == 4 || sg.G == VG) batch_block_chunk<Real, VG, true, DEEP>(sg, ch, lane, S, wait);
         else batch_block_chunk<Real, VG, false, DEEP>(sg, ch, lane, S, wait);
     }
@@ -349,26 +353,51 @@ __device__ __forceinline__ void batch_level_body(const BatchPlan &pl, uint32_t L
 // spills at 128 registers).  MINB: blocks per SM the
 // register allocation must allow (NoPivot: 4, at most 128 registers; FP32 deep
 // launches 5, at most 96).
-template <typename Real, bool ANY, int MINB = 1, bool DEEP = true>
+// SET: the classes it may meet, 1 those by vector width, 2 the direct one, 3 both
+// (together they take each other's registers).
+template <typename Real, bool ANY, int MINB = 1, bool DEEP = true, int SET = 1>
 __global__ void __launch_bounds__(128, MINB)
 batch_direct_level_kernel(const BatchSlot *__restrict__ slots, BatchPlan pl, uint32_t L, BatchCuts cut)
 {
     __shared__ BatchSeg sseg[kBatchSegWhole];
     static_assert(sizeof(sseg) >= sizeof(uint32_t) * kBatchSegSmem, "first chunks fit the staged segments' space");
-    __shared__ RecordStage<Real> stages[ANY ? 1 : 4];
-    RecordStage<Real> &S = stages[ANY ? 0 : threadIdx.x >> 5];
+    constexpr bool kStaged = !ANY && (SET & 1);
+    __shared__ RecordStage<Real> stages[kStaged ? 4 : 1];
+    RecordStage<Real> &S = stages[kStaged ? threadIdx.x >> 5 : 0];
     pdl_launch_dependents();
     bool waited = false;
     const uint32_t b = blockIdx.x;
-    if (b < cut.c[1]) {
-        batch_level_body<Real, 1, ANY, DEEP>(pl, L, 0, b, cut.c[1], sseg, S, waited);
-    } else if (b < cut.c[2]) {
-        batch_level_body<Real, 2, ANY, DEEP>(pl, L, 1, b - cut.c[1], cut.c[2] - cut.c[1], sseg, S, waited);
-    } else if constexpr (sizeof(Real) == 4) {
-        batch_level_body<Real, 4, ANY, DEEP>(pl, L, 2, b - cut.c[2], cut.c[3] - cut.c[2], sseg, S, waited);
+    if ((SET & 2) && (SET == 2 || b >= cut.c[kDirectClass])) {
+        constexpr int kVG = sizeof(Real) == 4 ? 4 : 2;
+        batch_level_body<Real, kVG, ANY, DEEP, true>(pl, L, kDirectClass, b - cut.c[kDirectClass],
+                                                     cut.c[kDirectClass + 1] - cut.c[kDirectClass], sseg, S, waited);
+    } else if constexpr (SET & 1) {
+        if (b < cut.c[1])
+            batch_level_body<Real, 1, ANY, DEEP, false>(pl, L, 0, b, cut.c[1], sseg, S, waited);
+        else if (b < cut.c[2])
+            batch_level_body<Real, 2, ANY, DEEP, false>(pl, L, 1, b - cut.c[1], cut.c[2] - cut.c[1], sseg, S, waited);
+        else if constexpr (sizeof(Real) == 4)
+            batch_level_body<Real, 4, ANY, DEEP, false>(pl, L, 2, b - cut.c[2], cut.c[3] - cut.c[2], sseg, S, waited);
     }
     if (!waited) pdl_wait_prerequisites();
     (void)slots;
+}
+
+// The NoPivot level kernel for the classes with blocks at this level.
+template <typename Real>
+const void *batch_level_fn(const BatchCuts &cut)
+{
+    constexpr bool f = sizeof(Real) == 4;
+    const bool direct = cut.c[kDirectClass + 1] > cut.c[kDirectClass], others = cut.c[kDirectClass] > 0;
+    if (direct && !others) return (const void *)batch_direct_level_kernel<Real, false, 4, true, 2>;
+    if constexpr (f) {
+        if (direct) return (const void *)batch_direct_level_kernel<Real, false, 4, false, 3>;
+        return batch_deep(cut) ? (const void *)batch_direct_level_kernel<Real, false, 5, true, 1>
+                               : (const void *)batch_direct_level_kernel<Real, false, 4, false, 1>;
+    } else {
+        return direct ? (const void *)batch_direct_level_kernel<Real, false, 4, true, 3>
+                      : (const void *)batch_direct_level_kernel<Real, false, 4, true, 1>;
+    }
 }
 
 template <typename Real, int VG, bool BLK, int NT, bool LEAN>
@@ -446,7 +475,7 @@ __device__ __noinline__ void batch_persist_class(const BatchPlan &pl, const Batc
         if (lane == 0) ch = atomicAdd(q, 1u);
         ch = __shfl_sync(0xffffffffu, ch, 0);
         if (ch >= nchunk) break;
-        batch_direct_chunk<Real, VG, ANY, kLoadL2>(segs, nseg, ch, lane, [] {});
+        batch_direct_chunk<Real, VG, ANY, kLoadL2, false>(segs, nseg, ch, lane, [] {});
     }
     __syncthreads();  // the segment list is restaged for the next class
 }

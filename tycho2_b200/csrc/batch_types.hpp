@@ -37,6 +37,7 @@ struct alignas(16) BatchSlot {
     uint32_t zero_row;     // psi's row of zeros (pass precision)
     uint32_t blk;          // block width of FP32 rows (0: plain)
     uint32_t turns;        // chain form: the block's warps take the levels in turn
+    uint32_t direct;       // level form: level_direct
     const uint32_t *chain_off;  // chain records: n_levels + 2 offsets per direction
 };
 
@@ -56,8 +57,9 @@ struct alignas(16) BatchSeg {
 };
 
 // Members are split by vector width (groups per psi-row access): class 0
-// = 1, class 1 = 2, class 2 = 4.
-constexpr uint32_t kBatchClasses = 3;
+// = 1, class 1 = 2, class 2 = 4; level_direct ones (FP64 pairs, FP32 fours) are
+// class 3.
+constexpr uint32_t kBatchClasses = 4, kDirectClass = 3;
 
 // Block ranges of one level launch: class c owns blocks [c[c], c[c+1]).
 struct BatchCuts {
@@ -89,7 +91,7 @@ cudaError_t launch_batch_psi_to_phi(bool fp32, const BatchSlot *slots, const Bat
                                     cudaStream_t s);
 cudaError_t launch_batch_post(const BatchSlot *slots, const BatchPlan &pl, unsigned grid, cudaStream_t s);
 cudaError_t launch_batch_finish(const BatchSlot *slots, const BatchPlan &pl, unsigned grid, cudaStream_t s);
-// One global level: cut.c[3] blocks of 4 warps (programmatic dependent launch);
+// One global level: cut.c[kBatchClasses] blocks of 4 warps (programmatic dependent launch);
 // any_solver: some member solves with Original or a Cramer solver (direct
 // kernel only; the shared-memory record kernels take NoPivot).
 template <typename Real>
