@@ -565,8 +565,8 @@ def run_large_leg(grp, dev, workload="kuhn64_s8_g16"):
     b32 = algorithmic_bytes(nc, A, G, info["n_incoming_interior"], 4)
     b64 = algorithmic_bytes(nc, A, G, info["n_incoming_interior"], 8)
     sw_shape32, sw_shape64 = sw.shape(1), sw.shape(0)
-    kern32 = kernel_name(sw_shape32, True, sw.launches(1))
-    kern64 = kernel_name(sw_shape64, False, sw.launches(0))
+    kern32 = kernel_name(sw_shape32, True, sw.launches(1) if sw_shape32["knob"] == 0 else None)
+    kern64 = kernel_name(sw_shape64, False, sw.launches(0) if sw_shape64["knob"] == 0 else None)
     tol, m = w.get("tol", 1e-10), w.get("restart", 30)
     phim, _, sm = sw.solve("mixed", iter_max=600, err_max=tol, restart=m, want_psi=False)
     phi64, _, s64 = sw.solve("gmres", iter_max=600, err_max=tol, restart=m, want_psi=False)

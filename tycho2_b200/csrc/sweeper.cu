@@ -395,6 +395,13 @@ int Sweeper::configure_default(int prec, std::string &err)
         gpv = block_rows_.groups / block_rows_.vg;
     }
     if (nc_ * gpv < (1ull << 26)) chains_[prec] = chain_shape(prec == 1, gpv == 1, items * gpv, A_);
+    // FP32 level launches over rows of four and more blocks of 4 groups: plain rows
+    // by the direct kernel, whose tasks of an item read side by side (24 lines of a
+    // warp's accesses a face, as blocks 32).  Sweep in ms, blocks / plain: 24^3 S8
+    // G=16 1.53 / 1.31, G=20 2.16 / 1.86, 32^3 S8 G=16 3.45 / 3.21, 16^3 S4 G=64 0.549 /
+    // 0.468, 24^3 S4 G=16 0.694 / 0.642; three blocks 24^3 S8 G=12 1.41 / 1.35, 24^3 S4
+    // G=12 0.727 / 0.778.
+    if (prec == 1 && vg == 4 && G_ >= 16 && !chains_[1].threads) block_[1] = false;
     return kOk;
 }
 
