@@ -210,9 +210,9 @@ constexpr uint32_t kBatchSegSmem = 256, kBatchSegWhole = 32;
 // One chunk (32 tasks of one member at one level) of the direct form: the
 // member's segment found by binary search, its compact record rebuilt in
 // registers, the source loaded, then (after `wait`, which the caller uses to
-// wait for the previous level) the upwind rows (read as MODE says; ALL: of the
-// four faces at once) and the solve.
-template <typename Real, int VG, bool ANY, int MODE, bool ALL, typename Wait>
+// wait for the previous level) the upwind rows (read as MODE says; of all four
+// faces at once) and the solve.
+template <typename Real, int VG, bool ANY, int MODE, bool FACTOR, typename Wait>
 __device__ __forceinline__ void batch_direct_chunk(const BatchSeg *segs, uint32_t nseg, uint32_t ch, uint32_t lane,
                                                    Wait wait)
 {
@@ -232,9 +232,10 @@ __device__ __forceinline__ void batch_direct_chunk(const BatchSeg *segs, uint32_
     const uint32_t g = (task - itl * gpv) * VG;
     RegRecord<Real> R;
     // NoPivot: the LU is rebuilt after the first upwind loads are issued, in
-    // their latency.
-    if constexpr (!ANY) load_compact_raw((const CompactRecord<Real> *)sg.rec + itl, R);
-    else load_record((const CompactRecord<Real> *)sg.rec + itl, R, p.solver);
+    // their latency; FACTOR false: with the record, before them.
+    constexpr bool kLate = !ANY && FACTOR;
+    if constexpr (kLate) load_compact_raw((const CompactRecord<Real> *)sg.rec + itl, R);
+    else load_record((const CompactRecord<Real> *)sg.rec + itl, R, ANY ? p.solver : (uint32_t)kSolveNoPivot);
     const bool live = R.u(0) != kSentinel;
     PairIn<Real, VG> in;
     if (live) pair_load_source<Real, VG>(p, R, g, in);
@@ -250,7 +251,7 @@ __device__ __forceinline__ void batch_direct_chunk(const BatchSeg *segs, uint32_
 #pragma unroll
                 for (int e = 0; e < VG; ++e) q[v][e] = in.q[v][e];
         };
-        sweep_task<Real, VG, MODE, true, ALL, false>(p, R, g, source);
+        sweep_task<Real, VG, MODE, FACTOR, true, false>(p, R, g, source);
     }
 }
 
@@ -475,7 +476,12 @@ __device__ __noinline__ void batch_persist_class(const BatchPlan &pl, const Batc
         if (lane == 0) ch = atomicAdd(q, 1u);
         ch = __shfl_sync(0xffffffffu, ch, 0);
         if (ch >= nchunk) break;
-        batch_direct_chunk<Real, VG, ANY, kLoadL2, false>(segs, nseg, ch, lane, [] {});
+        // all four faces at once, so that a chunk waits for the L2 once after its
+        // record; FP32 with the LU before them.  Pass of 256 uneven members by pairs
+        // of faces / so: FP32 58.2 / 49.4 ms, FP64 62.0 / 50.0 (51-65 from run to
+        // run); FP64 with the LU first 61.5, 24 members 3.99 / 3.96 and 4.65.
+        constexpr bool f = sizeof(Real) == 4;
+        batch_direct_chunk<Real, VG, ANY, kLoadL2, !f>(segs, nseg, ch, lane, [] {});
     }
     __syncthreads();  // the segment list is restaged for the next class
 }
