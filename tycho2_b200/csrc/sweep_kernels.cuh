@@ -71,8 +71,9 @@ __device__ __forceinline__ Real over12(Real x)
 
 // recip (nullable): the NoPivot pivots' reciprocals 1/M00, 1/a11, 1/b22,
 // computed by this function before (the FP64 compact records carry them),
-// used instead of dividing again.
-template <typename Real>
+// used instead of dividing again.  SKIP: branches around the faces that are not
+// outgoing.
+template <bool SKIP = false, typename Real>
 __device__ __forceinline__ void item_lu(ItemFactor<Real> &F, Real d1, Real d2, const bool (&out)[4],
                                         uint32_t kind = kSolveNoPivot, const Real *recip = nullptr);
 
@@ -254,7 +255,7 @@ __device__ __forceinline__ void factor16(const ItemFactor<Real> &F, uint32_t kin
 // The matrix of one (cell, angle) item from its face terms t1, t2 and the
 // volume terms d1 = sigma_t V/20, d2 = 2 sigma_t V/20 (out[f]: face f is
 // outgoing), and its LU factors.
-template <typename Real>
+template <bool SKIP, typename Real>
 __device__ __forceinline__ void item_lu(ItemFactor<Real> &F, Real d1, Real d2, const bool (&out)[4], uint32_t kind,
                                         const Real *recip)
 {
@@ -269,6 +270,7 @@ __device__ __forceinline__ void item_lu(ItemFactor<Real> &F, Real d1, Real d2, c
     // leaves every entry as it is and the code without branches.
 #pragma unroll
     for (int f = 0; f < 4; ++f) {
+        if (SKIP && !out[f]) continue;
         const Real o1 = out[f] ? F.t1[f] : Real(0), o2 = Real(2) * o1;
 #pragma unroll
         for (int i = 0; i < 4; ++i)
