@@ -1082,8 +1082,14 @@ sweep_direct_level_kernel(const LevelArgs p, const Rec *__restrict__ rec, const 
     RegRecord<Real> R;
     PairIn<Real, VG> in;
     constexpr bool kCompact = std::is_same<Rec, CompactRecord<Real>>::value;
-    // face-by-face tasks, except the packed FP32 form and the other solvers
-    constexpr bool kFaces = !ANY && !kPairedF32<Real, VG, ANY>;
+    // face-by-face tasks, except the packed FP32 form, the other solvers, and full
+    // FP64 records under a cap that those spill at, or loads wait at.  Sweep in ms,
+    // face by face / all upwind rows first: 20^3 S6 G=3 at 64 registers 0.90 / 0.80;
+    // at 85 20^3 S6 G=6 1.17 / 1.05, 16^3 S6 G=4 0.66 / 0.61, 24^3 S8 G=8 2.34 / 2.39; pairs of
+    // groups at 64 registers 24^3 S8 G=8 2.33 / 3.07.
+    constexpr bool kRowsFirst =
+        sizeof(Real) == 8 && !kCompact && (VG == 1 ? MINB != 1 && MINB != 10 : MINB == 12);
+    constexpr bool kFaces = !ANY && !kPairedF32<Real, VG, ANY> && !kRowsFirst;
     // Compact NoPivot records: the LU is rebuilt after the first upwind loads
     // are issued, in their latency.
     constexpr bool kLate = kCompact && !ANY && (kFaces || MINB == 1);
