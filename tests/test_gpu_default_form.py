@@ -23,7 +23,7 @@ CASES = [
     (13, 16, 2, 0, False),                          # and more than one of 512-thread ones
     (12, 8, 8, 0, False), (13, 6, 5, 1, None), (18, 8, 12, 1, False), (16, 8, 3, 0, False),
     (14, 8, 64, 0, False), (14, 8, 63, 0, False),   # deep launches: several runs per warp; the record prefetch
-    (5, 4, 16, 1, True), (18, 8, 16, 1, False), (18, 8, 20, 1, False), (12, 4, 64, 1, False),  # blocks in chains, else plain
+    (5, 4, 16, 1, True), (12, 4, 16, 1, False), (18, 8, 16, 1, False), (18, 8, 20, 1, False), (12, 4, 64, 1, False),  # blocks in chains, else plain
 ]
 
 

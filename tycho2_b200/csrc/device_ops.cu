@@ -443,9 +443,9 @@ inline unsigned blocks_for(uint64_t n, unsigned t = 256) { return (unsigned)((n 
 
 }  // namespace
 
-ChainShape chain_shape(bool fp32, bool one_block, double tasks, int directions)
+ChainShape chain_shape(bool fp32, bool one_block, double tasks, int directions, bool wide)
 {
-    return chain_shape_rule(fp32, one_block, tasks, directions);
+    return chain_shape_rule(fp32, one_block, tasks, directions, wide);
 }
 
 cudaError_t launch_item_abar(const uint32_t *items, uint64_t n, uint32_t A, const double *normal,

@@ -148,8 +148,8 @@ template <typename Real>
 cudaError_t launch_chains(ChainShape sh, const LevelArgs &p, const void *rec, const uint32_t *off, uint32_t n_levels,
                           uint32_t n_dir, cudaStream_t s);
 // The default form of a problem with so many tasks per level and direction;
-// one_block: rows of one block.
-ChainShape chain_shape(bool fp32, bool one_block, double tasks, int directions);
+// one_block: rows of one block; wide: FP32 rows of three and more blocks of 4.
+ChainShape chain_shape(bool fp32, bool one_block, double tasks, int directions, bool wide = false);
 // Persistent levels: one cooperative launch, a bounded grid barrier between
 // levels (level_off: device copy of the n_levels + 1 level offsets).
 template <typename Real>

@@ -242,14 +242,16 @@ cudaError_t launch_chains(ChainShape sh, const LevelArgs &p, const void *rec, co
 // 128) 283 / 197 / 189, (252, 72) 247 / 150 / 167, (327, 128) 643-674 / 531-566 /
 // 533-607, (640, 72) 352 / 349 / -, (655, 128) 909 / 1044 / 1261.  Up to 64 tasks 256
 // threads are as fast as 512 (128 a little slower), and more directions fit.
-inline ChainShape chain_shape_rule(bool fp32, bool one_block, double tasks, int directions)
+// Wide FP32 rows: (343, 32) 255 / 281 / -, (343, 8) 234 / 280, (345, 32) 344 / 390,
+// (303, 128) 188 / 166, (290, 72) 244 / 226.
+inline ChainShape chain_shape_rule(bool fp32, bool one_block, double tasks, int directions, bool wide)
 {
     const int sms = device_sm_count();
     ChainShape sh;
     if (tasks <= 64) {
         sh.threads = directions <= 2 * sms ? 256 : directions <= 4 * sms ? 128 : 0;
         sh.turns = true;
-    } else if (directions <= sms && tasks <= (fp32 ? 450 : one_block ? 340 : 200)) {
+    } else if (directions <= sms && tasks <= (wide ? 320 : fp32 ? 450 : one_block ? 340 : 200)) {
         sh.threads = 512;
         sh.turns = !fp32 || tasks <= 170;
     }

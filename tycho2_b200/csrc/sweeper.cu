@@ -394,7 +394,8 @@ int Sweeper::configure_default(int prec, std::string &err)
                                      (sizeof(float) * block_rows_.groups));
         gpv = block_rows_.groups / block_rows_.vg;
     }
-    if (nc_ * gpv < (1ull << 26)) chains_[prec] = chain_shape(prec == 1, gpv == 1, items * gpv, A_);
+    if (nc_ * gpv < (1ull << 26))
+        chains_[prec] = chain_shape(prec == 1, gpv == 1, items * gpv, A_, prec == 1 && vg == 4 && G_ >= 12);
     // FP32 level launches over rows of four and more blocks of 4 groups: plain rows
     // by the direct kernel, whose tasks of an item read side by side (24 lines of a
     // warp's accesses a face, as blocks 32).  Sweep in ms, blocks / plain: 24^3 S8
