@@ -116,7 +116,7 @@ batch_psi_to_phi_kernel(const BatchSlot *__restrict__ slots, BatchPlan pl)
         const uint32_t n = (uint32_t)((i1 + row - 1) / row - c0);
         if (n == 0) return;
         const PhiPlan plan = phi_plan<PhiBatch>((kPhiTile + row - 1) / row, row * (uint32_t)sizeof(Real), s.A);
-        phi_of_tiles<Real, PhiBatch>((const Real *)s.psi + c0 * s.A * row, s.w, n, s.A, row, plan, stages,
+        phi_of_tiles<Real, PhiBatch, false>((const Real *)s.psi + c0 * s.A * row, s.w, n, s.A, row, plan, stages,
                                      [&](uint32_t t0, uint32_t tn, const double (&v)[2]) {
             const uint32_t e = 2 * threadIdx.x;
             const uint64_t i = (c0 + t0) * row + e;

@@ -81,7 +81,7 @@ psi_to_phi_kernel(const Real *__restrict__ psi, const double *__restrict__ w, do
     pdl_wait_prerequisites();
     const uint64_t c0 = (uint64_t)blockIdx.x * plan.cells;
     const uint32_t row = 4 * Gp, n = (uint32_t)min((uint64_t)plan.cells, nc - c0);
-    phi_of_tiles<Real, Form>(psi + c0 * A * row, w, n, A, row, plan, stages,
+    phi_of_tiles<Real, Form, true>(psi + c0 * A * row, w, n, A, row, plan, stages,
                              [&](uint32_t, uint32_t, const double (&s)[Form::kElems]) {
 #pragma unroll
         for (int k = 0; k < Form::kElems; ++k) {

@@ -151,8 +151,9 @@ __host__ __device__ inline PhiPlan phi_plan(uint32_t cells, uint32_t row_bytes, 
 // E * threadIdx.x ... of the tile's (garbage beyond its end).  The stages of all
 // tiles are one sequence, so a tile's first ones are on their way while the tile
 // before is summed.  smem: the stages, each p.cells * p.stride bytes, 16-byte
-// aligned.  All threads of a block of Form::kThreads must call it.
-template <typename Real, typename Form, typename Emit>
+// aligned.  ONE: n <= p.cells.  All threads of a block of Form::kThreads must
+// call it.
+template <typename Real, typename Form, bool ONE, typename Emit>
 __device__ __forceinline__ void phi_of_tiles(const Real *__restrict__ psi, const double *__restrict__ w, uint32_t n,
                                              uint32_t A, uint32_t row, const PhiPlan &p, unsigned char *smem, Emit emit)
 {
@@ -165,8 +166,8 @@ __device__ __forceinline__ void phi_of_tiles(const Real *__restrict__ psi, const
     const unsigned char *src = reinterpret_cast<const unsigned char *>(psi) + (size_t)cell * A * rb;
     uint32_t ld_c0 = 0, ld_a0 = 0, ld_slot = 0;  // the next stage to load: its tile's first cell, first angle, place
     auto load = [&] {
-        if (ld_c0 < n) {
-            if (cell < p.cells && ld_c0 + cell < n) {
+        if (ONE ? ld_a0 < A : ld_c0 < n) {
+            if (ONE ? cell < n : cell < p.cells && ld_c0 + cell < n) {
                 const uint32_t bytes = min(p.angles, A - ld_a0) * rb;
                 unsigned char *d = smem + ld_slot * stage_bytes + cell * p.stride;
                 const unsigned char *q = src + (size_t)ld_a0 * rb;
@@ -174,7 +175,7 @@ __device__ __forceinline__ void phi_of_tiles(const Real *__restrict__ psi, const
             }
             ld_slot = ld_slot + 1 == NS ? 0 : ld_slot + 1;
             ld_a0 += p.angles;
-            if (ld_a0 >= A) {
+            if (!ONE && ld_a0 >= A) {
                 ld_a0 = 0;
                 ld_c0 += p.cells;
                 src += tile_bytes;
@@ -206,7 +207,8 @@ __device__ __forceinline__ void phi_of_tiles(const Real *__restrict__ psi, const
                 for (int k = 0; k < E; ++k) s[k] += (double)v.x[k] * wa;
             }
         }
-        emit(c0, min(p.cells, n - c0), s);
+        emit(c0, ONE ? n : min(p.cells, n - c0), s);
+        if (ONE) break;
     }
 }
 
