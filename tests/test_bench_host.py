@@ -83,3 +83,15 @@ def test_psi_hash_is_the_weighted_word_sum():
     want = sum(x * (2 * i + 1) for i, x in enumerate(words)) % (1 << 64)
     assert bench.psi_hash(psi) == "%016x" % want
     assert bench.psi_hash(psi, chunk=7) == "%016x" % want
+
+
+def test_reference_arm_is_the_reference_or_nothing(tmp_path, monkeypatch, capsys):
+    """Without the reference's own build, --impl reference says so instead of
+    timing the oracle's restatement under its name."""
+    import json
+    monkeypatch.setattr(bench, "REF_BIN", str(tmp_path))
+    monkeypatch.setattr(bench, "cpu_baseline", lambda *a, **k: pytest.fail("timed something else"))
+    monkeypatch.setattr(sys, "argv", ["bench.py", "--impl", "reference", "--gpus", "1"])
+    bench.main()
+    line = json.loads(capsys.readouterr().out)
+    assert line["impl"] == "reference" and line["unavailable"] and "value" not in line
