@@ -611,8 +611,9 @@ def run_parity(args, dev, cpu, gpu_psi_hash, phi_c2, sample, large, serve):
         out["c1"] = {"error": str(e)[:200]}
     c2 = {"workload": args.workload}
     if gpu_psi_hash and cpu and cpu.get("psi_hash"):
-        c2["fp64_sweep_bitexact_vs_reference"] = gpu_psi_hash == cpu["psi_hash"]
-        c2["psi_hash"] = {"gpu": gpu_psi_hash, "reference": cpu["psi_hash"]}
+        by = "reference" if cpu.get("kind") == "reference" else "oracle"
+        c2["fp64_sweep_bitexact_vs_" + by] = gpu_psi_hash == cpu["psi_hash"]
+        c2["psi_hash"] = {"gpu": gpu_psi_hash, by: cpu["psi_hash"]}
     if phi_c2:
         try:
             from oracle import kuhn_problem as kp

@@ -127,8 +127,9 @@ constexpr uint32_t block_width(uint32_t G) { return record_vg(true, G) == G ? 0u
 // Batched level launches: whether a member's rows stay plain with each thread
 // loading its record itself, instead of blocks and records by the warp's stage.
 // FP64 rows of several pairs (which are no blocks either way): pass in ms, staged /
-// direct, one 24^3 S4 member of 8 / 4 groups 1.09 / 1.05 and 0.876 / 0.81, four of 8
-// 3.25 / 3.00, one 24^3 S8 G=16 5.67 / 5.17; a row of one pair 28^3 S4 G=1 0.73 / 0.99.
+// direct, one 24^3 S4 member of 8 / 4 groups 1.14 / 1.08 and 0.905 / 0.837, four of 8
+// 3.29 / 3.05, one 24^3 S8 G=16 5.73 / 5.25; rows that are one block 28^3 S4 G=1 0.73 /
+// 0.99.
 // FP32 rows of three and more blocks: a face of four takes 32 lines of a warp's accesses as
 // blocks (two of 32 bytes a task), 24 plain (three of 16, the tasks of an item side
 // by side), of two blocks 32 and 48; two 24^3 S2 G=16 members 1.13 / 0.98, one 24^3 S4

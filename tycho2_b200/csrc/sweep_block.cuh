@@ -1,13 +1,15 @@
 // The default level kernel: 64-thread blocks, one (item, VG groups) task per
 // lane, compact records.
 //
-// What bounds a level kernel once a launch fills the GPU is the L1's line
-// lookups: an instruction looks up one line per cycle, and the lanes of a
-// warp read up to 32 different ones.  So this kernel makes fewer and wider
-// accesses than the direct ones (sweep_records.cuh):
+// What bounds a level kernel is its dependent loads through the L1, which takes
+// the up to 32 different lines of an instruction one after the other: a mid-sweep
+// FP32 launch keeps the L1 busy in 48% of the SM's cycles and waits for global
+// loads in 8 of 13.6 cycles per instruction; leaving the LU out of a sweep changes
+// it by less than 2%, the upwind loads by 30%.  So this kernel makes fewer and
+// wider accesses than the direct ones (sweep_records.cuh):
 //   * the warp copies its items' records, which are consecutive, as one run
-//     into shared memory (8 lookups for 16 FP32 records against 32, 7 for 8
-//     FP64 records against 49);
+//     into shared memory (8 lines for 16 FP32 records against 32, 7 for 8 FP64
+//     records against 49);
 //   * BLK: a task's values of a row, four vertices of VG groups, are one
 //     contiguous block, read and written by 32-byte accesses (two for 4 FP32
 //     groups instead of three per face and four per store; one for 1 or 2

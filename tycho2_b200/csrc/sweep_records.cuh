@@ -639,8 +639,7 @@ __device__ __forceinline__ const Real *face_row(const LevelArgs &p, const View &
     return reinterpret_cast<const Real *>(p.psi) + (uint64_t)at * (4u * p.G) + (BLK ? 4u * g : g);
 }
 
-// 32-byte accesses (sm_100): one instruction, so one line lookup of the L1,
-// where a 16-byte access takes two.
+// 32-byte accesses (sm_100): one instruction where 16-byte accesses are two.
 __device__ __forceinline__ void ld32(const float *p, float (&v)[8])
 {
     asm volatile("ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
@@ -837,10 +836,9 @@ __device__ __forceinline__ void solve_store_f32x2(const LevelArgs &p, const View
 // The LU is rebuilt in the first loads' latency; source(q) delivers the
 // sources.  The branch-free faces took the 4-group kernel at 85 registers
 // from about 640 to 356 executed instructions a task and from 20 bytes of
-// spills to none.  What bounds it then is the L1: each load instruction
-// looks up one line per cycle, and a warp's lanes touch up to 16 of them (at
-// 32^3 S8 G=8 a sweep of 2.12 ms keeps its 2.1 ms with the LU left out and
-// takes 1.47 ms without the upwind loads).
+// spills to none.  What bounds it then is its loads, whose lanes touch up to 16
+// lines an instruction (at 32^3 S8 G=8 a sweep of 2.12 ms keeps its 2.1 ms with the
+// LU left out and takes 1.47 ms without the upwind loads).
 template <int VG, int MODE, bool FACTOR, bool ALL, bool BLK, typename Source>
 __device__ __forceinline__ void task_f32x2(const LevelArgs &p, RegRecord<float> &R, uint32_t g, Source source)
 {
