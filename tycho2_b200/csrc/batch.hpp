@@ -43,9 +43,12 @@ struct BatchMemberStats {
 // chain against all levels as launches.  Measured on B200, us: a chain's
 // level 1.1 + k per task (k: FP64 0.0052 with 1 or 2 groups, 0.0085 with
 // more; FP32 0.0045); a level launch of the batch 2.7, and 15 tasks/ns.
-// FP32 pass in ms, chains / launches: one 24^3 S8 G=8 member 1.43 / 1.69
-// (estimates 1.02 / 1.42), one 24^3 S4 G=8 member 1.13 / 0.77 (1.02 / 0.68),
-// 24 uneven members 1.92 / 2.32 (0.54 / 2.59).
+// Pass in ms, chains / launches: FP32 one 24^3 S8 G=8 member 1.36 / 1.61 (the
+// estimates 1.02 / 1.42), one 24^3 S4 G=8 1.09 / 0.77 (1.02 / 0.68), one S6 1.19 / 1.12,
+// 24 uneven members 2.10 / 2.47 (0.54 / 2.59), 256 36.3 / 42.6; FP64 24 members 2.66 /
+// 3.42, 256 58.4 / 66.2, one 24^3 S6 G=8 2.17 / 1.77.  It takes launches where chains
+// would be faster for few FP64 members of several pairs: two 16^3 S6 G=4 0.61 / 0.78,
+// four 24^3 S4 G=8 2.86 / 3.03.
 class PassEstimate {
 public:
     double add(const Sweeper &sw, int prec);  // one member; its chains' time, us
