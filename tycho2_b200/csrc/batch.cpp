@@ -455,9 +455,12 @@ int Batch::build_graph(int prec, std::string &err)
             e = prec ? launch_batch_persist<float>(d_slots_[prec], plan, a, any_solver, st)
                      : launch_batch_persist<double>(d_slots_[prec], plan, a, any_solver, st);
     } else {
-        for (uint32_t L = 0; L < max_levels_ && e == cudaSuccess; ++L)
-            e = prec ? launch_batch_level<float>(ipw, d_slots_[prec], plan, L, cuts[L], any_solver, st)
-                     : launch_batch_level<double>(ipw, d_slots_[prec], plan, L, cuts[L], any_solver, st);
+        bool overlap = false;  // the first launch after the scattering source waits for all of it
+        for (uint32_t L = 0; L < max_levels_ && e == cudaSuccess; ++L) {
+            e = prec ? launch_batch_level<float>(ipw, d_slots_[prec], plan, L, cuts[L], any_solver, overlap, st)
+                     : launch_batch_level<double>(ipw, d_slots_[prec], plan, L, cuts[L], any_solver, overlap, st);
+            overlap = overlap || cuts[L].c[kBatchClasses] > 0;
+        }
     }
     if (e == cudaSuccess) e = launch_batch_psi_to_phi(prec == 1, d_slots_[prec], plan, kStreamGrid, st);
     if (e == cudaSuccess) e = launch_batch_post(d_slots_[prec], plan, kStreamGrid, st);

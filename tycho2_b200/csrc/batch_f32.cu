@@ -5,11 +5,11 @@
 namespace tycho {
 
 cudaError_t batch_level_launch(const void *fn, const BatchSlot *slots, const BatchPlan &pl, uint32_t level,
-                               const BatchCuts &cut, cudaStream_t s);
+                               const BatchCuts &cut, bool overlap, cudaStream_t s);
 
 template <>
 cudaError_t launch_batch_level<float>(int ipw, const BatchSlot *slots, const BatchPlan &pl, uint32_t level,
-                                      const BatchCuts &cut, bool any_solver, cudaStream_t s)
+                                      const BatchCuts &cut, bool any_solver, bool overlap, cudaStream_t s)
 {
     const void *fn = ipw == 0    ? (any_solver ? (const void *)batch_direct_level_kernel<float, true>
                                                : batch_level_fn<float>(cut))
@@ -18,7 +18,7 @@ cudaError_t launch_batch_level<float>(int ipw, const BatchSlot *slots, const Bat
                      : ipw == 32 ? (const void *)batch_level_kernel<float, 32>
                                  : nullptr;
     if (!fn) return cudaErrorInvalidValue;
-    return batch_level_launch(fn, slots, pl, level, cut, s);
+    return batch_level_launch(fn, slots, pl, level, cut, overlap, s);
 }
 
 template <>

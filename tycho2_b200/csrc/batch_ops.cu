@@ -199,7 +199,7 @@ __global__ void __launch_bounds__(256) batch_finish_kernel(const BatchSlot *__re
 }
 
 cudaError_t level_launch(const void *fn, const BatchSlot *slots, const BatchPlan &pl, uint32_t level,
-                         const BatchCuts &cut, cudaStream_t s)
+                         const BatchCuts &cut, bool overlap, cudaStream_t s)
 {
     const unsigned grid = cut.c[kBatchClasses];
     if (grid == 0) return cudaSuccess;
@@ -209,7 +209,7 @@ cudaError_t level_launch(const void *fn, const BatchSlot *slots, const BatchPlan
     cfg.stream = s;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[0].val.programmaticStreamSerializationAllowed = overlap;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     void *args[] = {(void *)&slots, (void *)&pl, (void *)&level, (void *)&cut};
@@ -219,14 +219,14 @@ cudaError_t level_launch(const void *fn, const BatchSlot *slots, const BatchPlan
 }  // namespace
 
 cudaError_t batch_level_launch(const void *fn, const BatchSlot *slots, const BatchPlan &pl, uint32_t level,
-                               const BatchCuts &cut, cudaStream_t s)
+                               const BatchCuts &cut, bool overlap, cudaStream_t s)
 {
-    return level_launch(fn, slots, pl, level, cut, s);
+    return level_launch(fn, slots, pl, level, cut, overlap, s);
 }
 
 template <>
 cudaError_t launch_batch_level<double>(int ipw, const BatchSlot *slots, const BatchPlan &pl, uint32_t level,
-                                       const BatchCuts &cut, bool any_solver, cudaStream_t s)
+                                       const BatchCuts &cut, bool any_solver, bool overlap, cudaStream_t s)
 {
     const void *fn = ipw == 0    ? (any_solver ? (const void *)batch_direct_level_kernel<double, true>
                                                : batch_level_fn<double>(cut))
@@ -235,7 +235,7 @@ cudaError_t launch_batch_level<double>(int ipw, const BatchSlot *slots, const Ba
                      : ipw == 32 ? (const void *)batch_level_kernel<double, 32>
                                  : nullptr;
     if (!fn) return cudaErrorInvalidValue;
-    return level_launch(fn, slots, pl, level, cut, s);
+    return level_launch(fn, slots, pl, level, cut, overlap, s);
 }
 
 // One block per SM up to three chains for each, else smaller ones: FP64 pass with

@@ -91,12 +91,14 @@ cudaError_t launch_batch_psi_to_phi(bool fp32, const BatchSlot *slots, const Bat
                                     cudaStream_t s);
 cudaError_t launch_batch_post(const BatchSlot *slots, const BatchPlan &pl, unsigned grid, cudaStream_t s);
 cudaError_t launch_batch_finish(const BatchSlot *slots, const BatchPlan &pl, unsigned grid, cudaStream_t s);
-// One global level: cut.c[kBatchClasses] blocks of 4 warps (programmatic dependent launch);
-// any_solver: some member solves with Original or a Cramer solver (direct
+// One global level: cut.c[kBatchClasses] blocks of 4 warps.  overlap: its blocks
+// may start while the kernel before it ends (programmatic dependent launch); they
+// read the source before they wait for that kernel, so it must be another level,
+// not the one that writes the source.  any_solver: some member solves with Original or a Cramer solver (direct
 // kernel only; the shared-memory record kernels take NoPivot).
 template <typename Real>
 cudaError_t launch_batch_level(int ipw, const BatchSlot *slots, const BatchPlan &pl, uint32_t level,
-                               const BatchCuts &cut, bool any_solver, cudaStream_t s);
+                               const BatchCuts &cut, bool any_solver, bool overlap, cudaStream_t s);
 // Threads of a chain's block in a pass of so many chains.
 int batch_chain_threads(size_t n_chains);
 // The wavefront of a pass as direction chains (compact records in chain
@@ -122,9 +124,9 @@ cudaError_t launch_batch_persist(const BatchSlot *slots, const BatchPlan &pl, co
                                  bool any_solver, cudaStream_t s);
 template <>
 cudaError_t launch_batch_level<double>(int ipw, const BatchSlot *slots, const BatchPlan &pl, uint32_t level,
-                                       const BatchCuts &cut, bool any_solver, cudaStream_t s);
+                                       const BatchCuts &cut, bool any_solver, bool overlap, cudaStream_t s);
 template <>
 cudaError_t launch_batch_level<float>(int ipw, const BatchSlot *slots, const BatchPlan &pl, uint32_t level,
-                                      const BatchCuts &cut, bool any_solver, cudaStream_t s);
+                                      const BatchCuts &cut, bool any_solver, bool overlap, cudaStream_t s);
 
 }  // namespace tycho
