@@ -11,7 +11,8 @@ import pytest
 pytestmark = pytest.mark.gpu
 
 CASES = [(1, 2, 1), (1, 4, 64), (2, 16, 1), (4, 4, 1), (9, 8, 1), (5, 6, 2), (4, 8, 3), (6, 6, 5), (7, 4, 7),
-         (8, 4, 8), (4, 10, 12), (3, 16, 16), (5, 4, 33), (4, 6, 63), (3, 8, 64)]
+         (8, 4, 8), (4, 10, 12), (3, 16, 16), (5, 4, 33), (4, 6, 63), (3, 8, 64),
+         (6, 4, 36), (4, 6, 40), (5, 4, 41)]
 
 
 def make(n, sn, G, fp32):

@@ -461,11 +461,12 @@ template <typename Real, typename Form>
 static cudaError_t launch_phi(const Real *psi, const double *w, double *phi, uint64_t nc, uint32_t A, uint32_t G,
                        uint32_t blk, uint32_t Gp, cudaStream_t s)
 {
-    // tiles of 256 elements; fewer cells a tile where those would not give
+    // tiles of an element or two per thread; fewer cells a tile where those would not give
     // every SM four blocks (8^3 of 4 elements: 512 tiles of 6 cells, not 48 of 64)
     const uint64_t blocks = 4 * (uint64_t)std::max(device_sm_count(), 1);
     const uint64_t even = (nc + blocks - 1) / blocks;
-    const PhiPlan plan = phi_plan<Form>((uint32_t)std::min<uint64_t>(kPhiTile / (4 * Gp), even),
+    const uint32_t tile = (uint32_t)Form::kElems * Form::kThreads;
+    const PhiPlan plan = phi_plan<Form>((uint32_t)std::min<uint64_t>(tile / (4 * Gp), even),
                                         4 * Gp * (uint32_t)sizeof(Real), A);
     const unsigned grid = (unsigned)((nc + plan.cells - 1) / plan.cells);
     void *args[] = {(void *)&psi, (void *)&w, (void *)&phi, (void *)&nc,  (void *)&A,
@@ -478,8 +479,12 @@ cudaError_t launch_psi_to_phi(const void *psi, bool psi_fp32, const double *w, d
                               uint64_t nc, uint32_t A, uint32_t G, uint32_t blk, uint32_t Gp, cudaStream_t s)
 {
     if (nc == 0) return cudaSuccess;
+    const uint32_t row = 4 * (psi_fp32 && blk ? Gp : G);
+    const bool wide = row > 128 && row <= 160;
+    if (!psi_fp32 && wide) return launch_phi<double, PhiWide>((const double *)psi, w, phi, nc, A, G, 0, G, s);
     if (!psi_fp32) return launch_phi<double, PhiOne>((const double *)psi, w, phi, nc, A, G, 0, G, s);
     if (G == 1) return launch_phi<float, PhiOne>((const float *)psi, w, phi, nc, A, G, blk, blk ? Gp : G, s);
+    if (wide) return launch_phi<float, PhiWide>((const float *)psi, w, phi, nc, A, G, blk, blk ? Gp : G, s);
     return launch_phi<float, PhiTwo>((const float *)psi, w, phi, nc, A, G, blk, blk ? Gp : G, s);
 }
 

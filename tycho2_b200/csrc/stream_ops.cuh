@@ -102,7 +102,7 @@ __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wai
 
 // Scalar flux, phi(c, v, g) = sum_a w_a psi(c, a, v, g), angles in increasing
 // order in FP64 (Util::psiToPhi, Util.cc:85-97), for tiles of whole cells (at
-// most 256 elements).  Bound by the bytes of psi, which a block streams
+// most 256 elements, wide ones 512).  Bound by the bytes of psi, which a block streams
 // through shared-memory stages, each some angles of each of its cells.  Loads
 // into registers, eight angles ahead of their sums, waited a memory latency
 // per eight angles: 32^3 S8, FP64 G=8 923 -> 906 us (7.1 TB/s), 24^3 G=3
@@ -112,9 +112,13 @@ __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wai
 // conversions and sums otherwise bound it (G=8 560 us), two elements per
 // thread of blocks of half as many threads, in 9 blocks with 2 stages of 8 KB.
 // At G=1 the second form's stages are a few angles of 64 cells: 169 us
-// against 105.
+// against 105.  Rows of 132 to 160 elements leave up to half of a 256-element
+// tile's threads idle; with two elements per thread of 256 a tile has three of
+// them (24^3 S4 G=33: FP32 405 -> 351 us, FP64 591 -> 487; G=40 at 20^3 FP64 375 -> 346;
+// G=48, rows of 192, FP32 20^3 S6 472 -> 499).
 struct PhiOne { static constexpr int kElems = 1, kThreads = 256, kStages = 4, kBytes = 12288; };
 struct PhiTwo { static constexpr int kElems = 2, kThreads = 128, kStages = 3, kBytes = 8192; };
+struct PhiWide { static constexpr int kElems = 2, kThreads = 256, kStages = 4, kBytes = 12288; };
 constexpr int kPhiTile = 256;
 
 struct PhiPlan {
